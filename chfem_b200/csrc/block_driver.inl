@@ -101,6 +101,18 @@ static bool launch_blk_apply(int parity, bool plain = false, int k0 = 0) {
   T* dold = (T*)(parity ? B->d1 : B->d0);
   T* dnew = (T*)(parity ? B->d0 : B->d1);
   const int precond = plain ? 0 : S->precond;
+  if (md_applies()) {
+    const int nb = md_block_ctas<ND, T>(NR, S->R, S->C, S->L, num_sms());
+    if (nb < 1) { set_err("block operator", "launch configuration"); return false; }
+    if (!ensure_reduction(nb)) return false;
+    const size_t off = (size_t)k0 * n;
+    TeArgs<ND, T> a{(const T*)B->r + off, dold + off, dnew + off, (T*)B->q + off, nullptr, nullptr, S->d_keys, nullptr, S->nmat, S->R, S->C, S->L,
+                    B->sc + k0, redctl(nb), FIN_ALPHA, 1, MrCfg{S->tol, 0, S->resnorm, precond, 0}};
+    const cudaError_t e = md_block_launch<ND, T>(NR, n, a, mddev<T>(), nb, S->stream);
+    S->launches++;
+    if (e != cudaSuccess) { set_err("block operator", cudaGetErrorString(e)); return false; }
+    return true;
+  }
   if (asm_applies()) return launch_asm_block<ND, T, NR>(dold, dnew, precond, k0);
   const dim3 block(TE_TR, TE_TC);
   if (!blk_prepare<ND, T, NR>()) return false;
@@ -282,8 +294,9 @@ static bool solve_block_device(const bool* has_x0) {
     if constexpr (NR == 6) {
       // once the first three cases (the normal strains, which converge first) are done, the
       // passes run on the last three only (the converged cases' lanes are no longer computed);
-      // a true-residual check that reopens one of the first three brings all six back
-      bool head_done = true;
+      // a true-residual check that reopens one of the first three brings all six back.  The
+      // pass in voxel modes deals its CTAs to the live right-hand sides itself.
+      bool head_done = !md_applies();
       for (int k = 0; k < 3; k++) head_done = head_done && B->h_sc[k].done;
       const int want = head_done ? 3 : 0;
       if (want != cur_k0) {

@@ -24,7 +24,7 @@
 #include "stencil_block.cuh"
 #include "stencil_asm.cuh"
 #include "asm_apply.h"
-#include "th_apply.h"
+#include "modal_apply.h"
 #include "stencil_2d.cuh"
 #include "pore_maps.h"
 #include "stencil_fluid_block.cuh"
@@ -117,11 +117,11 @@ struct Solver {
   // assembled neighbour blocks of a two-material model (stencil_asm.cuh), per precision
   double* d_tab64 = nullptr;
   float* d_tab32 = nullptr;
-  // thermal models with cubic-symmetric element matrices: the table of the thermal pass
-  // (stencil_th.cuh), per precision; th_state 0 not checked yet, 1 applies, -1 does not
-  double* d_th64 = nullptr;
-  float* d_th32 = nullptr;
-  int th_state = 0;
+  // 3D thermal / elastic models of isotropic materials: the table of the passes in voxel modes
+  // (stencil_modal.cuh), per precision; md_state 0 not checked yet, 1 applies, -1 does not
+  double* d_md64 = nullptr;
+  float* d_md32 = nullptr;
+  int md_state = 0;
   // scalar density field (cudapcgSetParametricDensityField): 16-bit code per voxel and its
   // range; the inverse Jacobi diagonal it implies, per unknown (FP64, built at solve set-up)
   uint16_t* d_sdf = nullptr;
@@ -248,12 +248,12 @@ static void free_model_dev() {
   if (!S) return;
   free_ptr(S->d_keys); free_ptr(S->d_dof_of_node); free_ptr(S->d_node_of_dof); free_ptr(S->d_bkeys);
   free_ptr(S->d_K64); free_ptr(S->d_K32); free_ptr(S->d_tab64); free_ptr(S->d_tab32);
-  free_ptr(S->d_th64); free_ptr(S->d_th32);
+  free_ptr(S->d_md64); free_ptr(S->d_md32);
   free_ptr(S->d_sdf); free_ptr(S->d_invd); free_ptr(S->d_img_fkeys);
   S->d_img_fkeys = nullptr; S->have_img_keys = false;
   S->d_keys = nullptr; S->d_dof_of_node = S->d_node_of_dof = nullptr; S->d_bkeys = nullptr;
   S->d_K64 = nullptr; S->d_K32 = nullptr; S->d_tab64 = nullptr; S->d_tab32 = nullptr;
-  S->d_th64 = nullptr; S->d_th32 = nullptr; S->th_state = 0;
+  S->d_md64 = nullptr; S->d_md32 = nullptr; S->md_state = 0;
   S->d_sdf = nullptr; S->d_invd = nullptr;
   S->have_K = S->have_keys = S->have_maps = false;
 }
@@ -326,9 +326,11 @@ static bool ensure_vectors() {
 }
 
 // Assembled neighbour blocks (stencil_asm.cuh) of a thermal/elastic model of at most two
-// materials; CHFEM_B200_BLOCK_OP=element keeps the element-by-element block operator.
+// materials that are not isotropic; CHFEM_B200_BLOCK_OP=element keeps the element-by-element
+// operator.
+static bool md_applies();
 static bool asm_applies() {
-  if (S->fluid || S->dim2 || S->nmat > 2 || S->d_sdf) return false;
+  if (S->fluid || S->dim2 || S->nmat > 2 || S->d_sdf || md_applies()) return false;
   const char* e = getenv("CHFEM_B200_BLOCK_OP");
   return !(e && !strcmp(e, "element"));
 }
@@ -350,32 +352,33 @@ static bool ensure_tab() {
   return true;
 }
 
-// The thermal pass of stencil_th.cuh: 3D thermal models without a density field whose element
-// matrices have the cubic structure it relies on (checked once per model);
-// CHFEM_B200_THERMAL_OP=generic keeps the generic pass.
-static bool th_applies() {
-  if (S->analysis != CUDAPCG_THERMAL_3D || S->d_sdf || S->nmat > 4 || !S->have_K) return false;
-  const char* e = getenv("CHFEM_B200_THERMAL_OP");
-  if (e && !strcmp(e, "generic")) return false;
-  if (S->th_state == 0) {
-    std::vector<double> t((size_t)th_table_words());
-    S->th_state = th_build_table((int)S->nmat, S->Kd.data(), t.data()) ? 1 : -1;
+// The passes in voxel modes (stencil_modal.cuh): 3D thermal and elastic models whose element
+// matrices are those of isotropic materials on cubes (checked once per model), the reference's
+// and this library's models.  CHFEM_B200_THERMAL_OP=generic (thermal) and
+// CHFEM_B200_BLOCK_OP=element (elastic) keep the passes that take any element matrix.
+static bool md_applies() {
+  if (S->fluid || S->dim2 || S->nmat > 4 || !S->have_K || !md_layer_fits(S->nd, S->R, S->C)) return false;
+  const char* e = getenv(S->nd == 1 ? "CHFEM_B200_THERMAL_OP" : "CHFEM_B200_BLOCK_OP");
+  if (e && !strcmp(e, S->nd == 1 ? "generic" : "element")) return false;
+  if (S->md_state == 0) {
+    std::vector<double> t((size_t)md_table_words());
+    S->md_state = md_build_table(S->nd, S->nmat, S->Kd.data(), t.data()) ? 1 : -1;
   }
-  return S->th_state == 1;
+  return S->md_state == 1;
 }
-template <typename T> static T*& thdev();
-template <> double*& thdev<double>() { return S->d_th64; }
-template <> float*& thdev<float>() { return S->d_th32; }
+template <typename T> static T*& mddev();
+template <> double*& mddev<double>() { return S->d_md64; }
+template <> float*& mddev<float>() { return S->d_md32; }
 template <typename T>
-static bool ensure_th() {
-  if (thdev<T>()) return true;
-  std::vector<double> t64((size_t)th_table_words());
-  if (!th_build_table((int)S->nmat, S->Kd.data(), t64.data())) { set_err("solve", "thermal table"); return false; }
+static bool ensure_md() {
+  if (mddev<T>()) return true;
+  std::vector<double> t64((size_t)md_table_words());
+  if (!md_build_table(S->nd, S->nmat, S->Kd.data(), t64.data())) { set_err("solve", "table of the voxel modes"); return false; }
   std::vector<T> t(t64.begin(), t64.end());
   T* d = nullptr;
   CKV(dev_malloc(&d, t.size() * sizeof(T)));
   CKV(cudaMemcpy(d, t.data(), t.size() * sizeof(T), cudaMemcpyHostToDevice));
-  thdev<T>() = d;
+  mddev<T>() = d;
   return true;
 }
 
@@ -435,7 +438,7 @@ template <> float* Kdev<float>() { return S->d_K32; }
 template <typename T>
 static bool ensure_K() {
   if (Kdev<T>()) {  // the derived tables may have been dropped since (new density field, new model)
-    if (th_applies() && !ensure_th<T>()) return false;
+    if (md_applies() && !ensure_md<T>()) return false;
     if (asm_applies() && !ensure_tab<T>()) return false;
     if ((S->d_sdf || S->dim2) && !ensure_invd()) return false;
     return true;
@@ -447,7 +450,7 @@ static bool ensure_K() {
   CKV(dev_malloc(&dk, kt.size() * sizeof(T)));
   CKV(cudaMemcpy(dk, kt.data(), kt.size() * sizeof(T), cudaMemcpyHostToDevice));
   if (sizeof(T) == 8) S->d_K64 = (double*)dk; else S->d_K32 = (float*)dk;
-  if (th_applies() && !ensure_th<T>()) return false;
+  if (md_applies() && !ensure_md<T>()) return false;
   if (asm_applies() && !ensure_tab<T>()) return false;
   if ((S->d_sdf || S->dim2) && !ensure_invd()) return false;
   if (S->fluid) {
@@ -517,6 +520,19 @@ static int d2_ctas() {
   return (int)std::max(1L, std::min(tiles, 8L * num_sms()));
 }
 
+// One operator pass in voxel modes (md_applies) on explicit buffers, with the scalars of S->cur_sc.
+template <int ND, typename T, int MODE>
+static bool launch_md(const T* in0, const T* in1, T* vout, T* y, double* x, const T* d, int finish, int skip_if_done, const MrCfg& cfg) {
+  const int nb = md_ctas<ND, T, MODE>(S->d_sdf != nullptr, S->R, S->C, S->L, num_sms());
+  if (nb < 1 || !ensure_reduction(nb)) return false;
+  TeArgs<ND, T> a{in0, in1, vout, y, x, d, S->d_keys, nullptr, S->nmat, S->R, S->C, S->L, S->cur_sc, redctl(nb), finish, skip_if_done, cfg};
+  sdf_args(a);
+  const cudaError_t e = md_launch<ND, T, MODE>(a, mddev<T>(), nb, S->stream);
+  S->launches++;
+  if (e != cudaSuccess) { set_err("operator pass", cudaGetErrorString(e)); return false; }
+  return true;
+}
+
 template <typename T>
 static bool launch_apply(const T* in0, const T* in1, T* vout, T* y, bool fuse, int finish, bool skip_if_done) {
   if (S->fluid) {
@@ -551,14 +567,11 @@ static bool launch_apply(const T* in0, const T* in1, T* vout, T* y, bool fuse, i
       if (fuse) k_2d_apply<2, T, TE_PCG><<<nb, dim3(T2_TR, T2_TC), t2_smem_bytes<2, T>(), S->stream>>>(a);
       else k_2d_apply<2, T, TE_PLAIN><<<nb, dim3(T2_TR, T2_TC), t2_smem_bytes<2, T>(), S->stream>>>(a);
     }
-  } else if (th_applies()) {
-    const int nb = fuse ? th_ctas<T, TE_PCG>(S->R, S->C, S->L, num_sms()) : th_ctas<T, TE_PLAIN>(S->R, S->C, S->L, num_sms());
-    if (nb < 1 || !ensure_reduction(nb)) return false;
-    TeArgs<1, T> a{in0, in1, vout, y, nullptr, nullptr, S->d_keys, Kdev<T>(), S->nmat, S->R, S->C, S->L, S->cur_sc, redctl(nb), finish, skip_if_done, MrCfg{S->tol, 0, S->resnorm, S->precond, 0}};
-    const cudaError_t e = fuse ? th_launch<T, TE_PCG>(a, thdev<T>(), nb, S->stream) : th_launch<T, TE_PLAIN>(a, thdev<T>(), nb, S->stream);
-    S->launches++;
-    if (e != cudaSuccess) { set_err("operator pass", cudaGetErrorString(e)); return false; }
-    return true;
+  } else if (md_applies()) {
+    if (S->nd == 1) return fuse ? launch_md<1, T, TE_PCG>(in0, in1, vout, y, nullptr, nullptr, finish, skip_if_done, MrCfg{S->tol, 0, S->resnorm, S->precond, 0})
+                                : launch_md<1, T, TE_PLAIN>(in0, in1, vout, y, nullptr, nullptr, finish, skip_if_done, MrCfg{S->tol, 0, S->resnorm, S->precond, 0});
+    return fuse ? launch_md<3, T, TE_PCG>(in0, in1, vout, y, nullptr, nullptr, finish, skip_if_done, MrCfg{S->tol, 0, S->resnorm, S->precond, 0})
+                : launch_md<3, T, TE_PLAIN>(in0, in1, vout, y, nullptr, nullptr, finish, skip_if_done, MrCfg{S->tol, 0, S->resnorm, S->precond, 0});
   } else if (asm_applies()) {
     int nb;
     cudaError_t e;
@@ -664,11 +677,9 @@ static bool launch_te_mode(const T* in0, const T* in1, T* vout, double* x, int f
       k_2d_apply<2, T, MODE><<<nb, dim3(T2_TR, T2_TC), t2_smem_bytes<2, T>(), S->stream>>>(a);
     }
     e = cudaGetLastError();
-  } else if (th_applies()) {
-    const int nb = th_ctas<T, MODE>(S->R, S->C, S->L, num_sms());
-    if (nb < 1 || !ensure_reduction(nb)) return false;
-    TeArgs<1, T> a{in0, in1, vout, nullptr, x, nullptr, S->d_keys, Kdev<T>(), S->nmat, S->R, S->C, S->L, S->cur_sc, redctl(nb), finish, 1, cfg};
-    e = th_launch<T, MODE>(a, thdev<T>(), nb, S->stream);
+  } else if (md_applies()) {
+    return S->nd == 1 ? launch_md<1, T, MODE>(in0, in1, vout, nullptr, x, nullptr, finish, 1, cfg)
+                      : launch_md<3, T, MODE>(in0, in1, vout, nullptr, x, nullptr, finish, 1, cfg);
   } else if (asm_applies()) {
     if (S->nd == 1) {
       const int nb = asm_te_ctas<1, T, MODE>(S->R, S->C, S->L, num_sms());
@@ -1409,7 +1420,7 @@ cudapcgFlag_t cudapcgSetParametricDensityField(parametricScalarField_t* field, d
   }
   free_ptr(S->d_invd); S->d_invd = nullptr;
   free_ptr(S->d_tab64); free_ptr(S->d_tab32); S->d_tab64 = nullptr; S->d_tab32 = nullptr;
-  free_ptr(S->d_th64); free_ptr(S->d_th32); S->d_th64 = nullptr; S->d_th32 = nullptr; S->th_state = 0;
+  free_ptr(S->d_md64); free_ptr(S->d_md32); S->d_md64 = nullptr; S->d_md32 = nullptr; S->md_state = 0;
   invalidate_graphs();
   return CUDAPCG_TRUE;
 }
@@ -1503,7 +1514,7 @@ cudapcgFlag_t cudapcgSetLclMtxs(cudapcgVar_t* Lm) {
   S->have_K = true;
   free_ptr(S->d_K64); free_ptr(S->d_K32); S->d_K64 = nullptr; S->d_K32 = nullptr;
   free_ptr(S->d_tab64); free_ptr(S->d_tab32); S->d_tab64 = nullptr; S->d_tab32 = nullptr;
-  free_ptr(S->d_th64); free_ptr(S->d_th32); S->d_th64 = nullptr; S->d_th32 = nullptr; S->th_state = 0;
+  free_ptr(S->d_md64); free_ptr(S->d_md32); S->d_md64 = nullptr; S->d_md32 = nullptr; S->md_state = 0;
   free_ptr(S->d_invd); S->d_invd = nullptr;
   invalidate_graphs();  // captured launches hold the old matrix pointers
   if (S->fluid && !set_fluid_diag()) return CUDAPCG_FALSE;

@@ -70,7 +70,10 @@ struct TeWork {
   __device__ TeWork(int R, int C, int L_, int tc_ = TE_TC) : tiles_r((R + TE_TR - 1) / TE_TR), L(L_), tc(tc_) {
     tiles = (long)tiles_r * ((C + tc - 1) / tc);
     W = tiles * L;
-    const long P = gridDim.x;
+    share(gridDim.x);
+  }
+  // the line cut for P CTAs (the constructor: the whole grid)
+  __device__ void share(long P) {
     lc = (int)min((long)L, max(1L, (W + P - 1) / P));
     nc = (L + lc - 1) / lc;
   }
