@@ -130,6 +130,11 @@ template <int ND, typename T, int NR>
 static bool launch_blk_point(int parity, int k0 = 0) {
   const long n = S->nvars;
   T* dnew = (T*)(parity ? B->d0 : B->d1);
+  if (md_applies()) {
+    const size_t off = (size_t)k0 * n;
+    return launch_md_point<T>(NR, B->x + off, dnew + off, (const T*)(parity ? B->d1 : B->d0) + off, (T*)B->r + off, (const T*)B->q + off,
+                              B->sc + k0, parity);
+  }
   // whole 16-byte chunks per thread when every right-hand side's vectors start aligned
   const bool chunks = n % 4 == 0;
   const int g = pw_grid(chunks ? n / 4 : S->N);
@@ -169,8 +174,8 @@ static double time_block_kernel_T(int which, unsigned reps) {
     cudaMemcpyAsync(B->sc, B->h_sc, nr * sizeof(DevScalars), cudaMemcpyHostToDevice, S->stream);
     cudaEventRecord(S->ev0, S->stream);
     bool ok;
-    if (S->nd == 1) ok = which == 5 ? launch_blk_apply<1, T, 3>(0) : launch_blk_point<1, T, 3>(0);
-    else ok = which == 5 ? launch_blk_apply<3, T, 6>(0) : launch_blk_point<3, T, 6>(0);
+    if (S->nd == 1) ok = which == 5 ? launch_blk_apply<1, T, 3>(0) : launch_blk_point<1, T, 3>(1);
+    else ok = which == 5 ? launch_blk_apply<3, T, 6>(0) : launch_blk_point<3, T, 6>(1);
     cudaEventRecord(S->ev1, S->stream);
     if (!ok || cudaEventSynchronize(S->ev1) != cudaSuccess) return -1.0;
     float ms = 0;

@@ -45,6 +45,7 @@ struct DevScalars {
   double res0;       // stopping reference for the INF / PMINRES norms
   double metric;     // last stopping metric
   double red[6];     // scratch results of the last reductions
+  double xa;         // step not yet added to x (k_md_point): x lacks xa times the previous direction
   int iteration;
   int done;          // 1 once the stopping test passed or max iterations were reached
   int found;         // 1 when the stopping test passed

@@ -25,6 +25,7 @@
 #include "stencil_asm.cuh"
 #include "asm_apply.h"
 #include "modal_apply.h"
+#include "modal_point.cuh"
 #include "stencil_2d.cuh"
 #include "pore_maps.h"
 #include "stencil_fluid_block.cuh"
@@ -728,11 +729,26 @@ static bool enqueue_pcg3_iteration(int parity) {
          launch_te_mode<T, TE_UPD>(dnew, nullptr, (T*)S->r, S->x, FIN_STORE);
 }
 
+// The pointwise PCG pass of models whose operator runs in voxel modes (modal_point.cuh), on nr
+// right-hand sides with the scalar records sc.
+template <typename T>
+static bool launch_md_point(int nr, double* x, const T* d, const T* dold, T* r, const T* q, DevScalars* sc, int parity) {
+  const int nb = md_point_ctas(S->nvars, num_sms());
+  if (!ensure_reduction(nb)) return false;
+  const MdPw<T> a{x, d, dold, r, q, S->d_keys, mddev<T>(), S->d_invd, S->nmat, S->nvars, sc, redctl(nb), solvecfg()};
+  const bool norms = S->resnorm != CUDAPCG_L2_NORM;
+  const cudaError_t e = S->nd == 1 ? md_point_launch<1, T>(nr, a, parity, norms, nb, S->stream) : md_point_launch<3, T>(nr, a, parity, norms, nb, S->stream);
+  S->launches++;
+  if (e != cudaSuccess) { set_err("pointwise pass", cudaGetErrorString(e)); return false; }
+  return true;
+}
+
 template <typename T>
 static bool enqueue_pcg_iteration(int parity) {
   T* dold = (T*)(parity ? S->d1 : S->d0);
   T* dnew = (T*)(parity ? S->d0 : S->d1);
   if (!launch_apply<T>(pcg_dir_in<T>(), dold, dnew, (T*)S->q, true, FIN_ALPHA, true)) return false;
+  if (md_applies()) return launch_md_point<T>(1, S->x, dnew, dold, (T*)S->r, (const T*)S->q, S->cur_sc, parity);
   return launch_point<T, PW_PCG>(S->x, dnew, (T*)S->r, (const T*)S->q, s_or_null<T>(), nullptr);
 }
 
@@ -1675,7 +1691,10 @@ static double time_kernel_T(int which, unsigned reps) {
     switch (which) {
       case 0: ok = launch_apply<T>((const T*)S->d0, nullptr, nullptr, (T*)S->q, false, FIN_NONE, false); break;
       case 1: ok = launch_apply<T>(pcg_dir_in<T>(), (const T*)S->d0, (T*)S->d1, (T*)S->q, true, FIN_ALPHA, false); break;
-      case 2: ok = launch_point<T, PW_PCG>(S->x, (T*)S->d1, (T*)S->r, (const T*)S->q, s_or_null<T>(), nullptr); break;
+      case 2:
+        ok = md_applies() ? launch_md_point<T>(1, S->x, (const T*)S->d0, (const T*)S->d1, (T*)S->r, (const T*)S->q, S->d_sc, 1)
+                          : launch_point<T, PW_PCG>(S->x, (T*)S->d1, (T*)S->r, (const T*)S->q, s_or_null<T>(), nullptr);
+        break;
       case 3: ok = launch_mr_op<T>((const T*)S->r, (T*)S->r2, FIN_MR_STEP, false); break;
       case 4: ok = launch_mr_dir<T>((const T*)S->r); break;
       default: ok = false;

@@ -5,6 +5,7 @@
 #include <vector>
 #include "modal_apply.h"
 #include "stencil_modal.cuh"
+#include "modal_point.cuh"
 
 namespace chfem {
 
@@ -170,5 +171,36 @@ CHFEM_MD_BLOCK(1, float)
 CHFEM_MD_BLOCK(1, double)
 CHFEM_MD_BLOCK(3, float)
 CHFEM_MD_BLOCK(3, double)
+
+// CTAs of 256 threads: 4 per SM keep enough 16-byte loads in flight for the memory's latency and
+// the partials that the last CTA sums few.
+int md_point_ctas(long n, int num_sms) { return (int)std::max(1L, std::min(4L * num_sms, (n / 2 + MP_NT - 1) / MP_NT)); }
+
+namespace {
+template <int ND, typename T, int NR, int VW>
+void point(const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st) {
+  if (norms) k_md_point<ND, T, NR, 2, VW><<<nb, MP_NT, 0, st>>>(a);
+  else if (parity) k_md_point<ND, T, NR, 1, VW><<<nb, MP_NT, 0, st>>>(a);
+  else k_md_point<ND, T, NR, 0, VW><<<nb, MP_NT, 0, st>>>(a);
+}
+template <int ND, typename T, int NR>
+void point_width(const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st) {
+  constexpr int FULL = 16 / (int)sizeof(T);
+  if (NR == 1 || a.n % FULL == 0) point<ND, T, NR, FULL>(a, parity, norms, nb, st);
+  else if (FULL == 4 && a.n % 2 == 0) point<ND, T, NR, 2>(a, parity, norms, nb, st);
+  else point<ND, T, NR, 1>(a, parity, norms, nb, st);
+}
+}  // namespace
+template <int ND, typename T>
+cudaError_t md_point_launch(int nr, const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st) {
+  if (nr == 1) point_width<ND, T, 1>(a, parity, norms, nb, st);
+  else if (nr == 3) point_width<ND, T, 3>(a, parity, norms, nb, st);
+  else if constexpr (ND == 3) point_width<ND, T, 6>(a, parity, norms, nb, st);
+  return cudaGetLastError();
+}
+template cudaError_t md_point_launch<1, float>(int, const MdPw<float>&, int, bool, int, cudaStream_t);
+template cudaError_t md_point_launch<1, double>(int, const MdPw<double>&, int, bool, int, cudaStream_t);
+template cudaError_t md_point_launch<3, float>(int, const MdPw<float>&, int, bool, int, cudaStream_t);
+template cudaError_t md_point_launch<3, double>(int, const MdPw<double>&, int, bool, int, cudaStream_t);
 
 }  // namespace chfem

@@ -28,4 +28,13 @@ int md_block_ctas(int nr, int R, int C, int L, int num_sms);
 template <int ND, typename T>
 cudaError_t md_block_launch(int nr, long n, const TeArgs<ND, T>& a, const T* tab, int nb, cudaStream_t st);
 
+// The pointwise PCG pass (modal_point.cuh) on nr right-hand sides, n unknowns apart; parity: which
+// pass of a pair (x is updated in the second), norms: the stopping test reads max-norms (x is
+// updated in every pass).
+template <typename T>
+struct MdPw;
+int md_point_ctas(long n, int num_sms);
+template <int ND, typename T>
+cudaError_t md_point_launch(int nr, const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st);
+
 }  // namespace chfem

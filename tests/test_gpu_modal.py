@@ -83,13 +83,15 @@ def test_solve_equals_general_pass(tmp_path, monkeypatch, analysis, shape, nmat,
         assert lib.cudapcgSetNumTol(tol) and lib.cudapcgSetMaxIterations(20000) and lib.cudapcgAllocateArrays()
         assert lib.cudapcgSetRHS(ptr(b))
         x = np.zeros(a["ndof"])
-        assert lib.cudapcgSolve(ptr(x)), lib.cudapcgB200LastError()
+        # under the error norm CG may stop on the residual first, which reports "not found"
+        found = lib.cudapcgSolve(ptr(x))
+        assert (found or norm == 2) and not lib.cudapcgB200LastError(), lib.cudapcgB200LastError()
         its = lib.cudapcgGetNumIterations()
         lib.cudapcgEnd()
         x -= np.tile(x.reshape(-1, dof).mean(axis=0), a["ndof"] // dof)
         return x, its
     (x, its), (xref, itsref) = both(monkeypatch, analysis, run)
-    assert abs(its - itsref) <= 1
+    assert abs(its - itsref) <= 1 and its < 20000
     # the error norm bounds the last step instead of the residual: the iterates of one count
     assert H.rel_to_max(x, xref) < (10 * tol if its == itsref else 1e-4)
 
