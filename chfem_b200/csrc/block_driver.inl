@@ -8,6 +8,7 @@ struct BlockState {
   long n = 0;
   void *r = nullptr, *s = nullptr, *d0 = nullptr, *d1 = nullptr, *q = nullptr;  // [nr][n], work precision
   double *x = nullptr, *b64 = nullptr;                                          // [nr][n], FP64
+  double* z = nullptr;        // Stokes: the records of z = M^-1 r, [nV + nB][nr][4]
   DevScalars* sc = nullptr;   // [nr]
   DevScalars* h_sc = nullptr; // pinned [nr]
   double* d_mom = nullptr;    // load-case moments [BLK_MAX][8] + CB staging
@@ -22,7 +23,7 @@ static void block_invalidate() {
 
 static void block_free() {
   if (!B) return;
-  void* ps[] = {B->r, B->s, B->d0, B->d1, B->q, B->x, B->b64, B->sc, B->d_mom};
+  void* ps[] = {B->r, B->s, B->d0, B->d1, B->q, B->x, B->b64, B->z, B->sc, B->d_mom};
   for (void* p : ps) free_ptr(p);
   if (B->h_sc) cudaFreeHost(B->h_sc);
   if (B->gexec) cudaGraphExecDestroy(B->gexec);
@@ -39,9 +40,10 @@ static bool block_alloc(int nr) {
   B->nr = nr; B->prec = p; B->n = S->nvars;
   const size_t tot = (size_t)nr * std::max<long>(S->nvars, 1);
   // thermal / elastic: r, the direction's two buffers and q (s = M^-1 r is formed by the
-  // operator pass); Stokes (P)MINRES also keeps s
-  std::vector<void**> vs = {&B->r, &B->d0, &B->d1, &B->q};
-  if (S->fluid) vs.push_back(&B->s);
+  // operator pass); Stokes (P)MINRES: r, d, q, s = A M^-1 r and z
+  std::vector<void**> vs = {&B->r, &B->d0, &B->q};
+  vs.push_back(S->fluid ? &B->s : &B->d1);
+  if (S->fluid) CKV(dev_malloc(&B->z, (size_t)(S->nV + S->nB) * nr * 4 * 8));
   for (void** v : vs) { CKV(dev_malloc(v, tot * sizeof(T))); CKV(cudaMemset(*v, 0, tot * sizeof(T))); }
   CKV(dev_malloc(&B->x, tot * 8));
   CKV(dev_malloc(&B->b64, tot * 8));
@@ -324,30 +326,13 @@ static bool solve_block_device(const bool* has_x0) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Block (P)MINRES for the Stokes flow directions.  Buffers: r and r' alternate between
-// B->r and B->d1, the direction is B->d0, q = A d is B->q, s = A M^-1 r is B->s.
-template <typename T, int NR>
-static bool launch_fl_blk_dir(int parity) {
-  const T* rcur = (const T*)(parity ? B->d1 : B->r);
-  const int g = pw_grid(S->nV + S->nB);
-  if (!ensure_reduction(g)) return false;
-  FlBlkDir<T> a{(T*)B->d0, (T*)B->q, rcur, (const T*)B->s, S->d_bkeys, S->nV, S->nB, S->nvars, B->sc, redctl(g), S->precond};
-  k_fl_blk_dir<T, NR><<<g, PW_NT, 0, S->stream>>>(a);
-  S->launches++;
-  return cudaPeekAtLastError() == cudaSuccess;
-}
-template <typename T, int NR>
-static bool launch_fl_blk_apply(int parity) {
-  const T* rcur = (const T*)(parity ? B->d1 : B->r);
-  T* rnext = (T*)(parity ? B->r : B->d1);
-  const int g = pw_grid(S->nV + S->nB);
-  if (!ensure_reduction(g)) return false;
-  FlBlkArgs<T> a{rcur, (const T*)B->q, rnext, (T*)B->s, B->x, (const T*)B->d0, S->d_dof_of_node, S->d_node_of_dof, S->d_bkeys,
-                 S->R, S->C, S->L, S->nV, S->nB, S->nvars, B->sc, redctl(g), mrcfg()};
-  if (S->resnorm == CUDAPCG_L2_NORM) k_fl_blk_apply<T, NR, false><<<g, FL_NT, 0, S->stream>>>(a);
-  else k_fl_blk_apply<T, NR, true><<<g, FL_NT, 0, S->stream>>>(a);
-  S->launches++;
-  return cudaPeekAtLastError() == cudaSuccess;
+// Block (P)MINRES for the Stokes flow directions (stencil_fluid_mr.cuh): direction B->d0,
+// q = A d B->q, s = A M^-1 r B->s, z = M^-1 r B->z; r is updated in place.
+template <int NR>
+static bool enqueue_fl_blk_iteration() {
+  FlMrArgs a = fl_mr_args((double*)B->r, (double*)B->q, (double*)B->s, (double*)B->d0, B->x, B->z, FIN_MR_STEP, true);
+  a.sc = B->sc;
+  return launch_fl_mr_dir<NR>(a) && launch_fl_mr_upd<NR>(a) && launch_fl_mr_apply<NR>(a);
 }
 
 template <typename T, int NR>
@@ -359,7 +344,7 @@ static bool blk_build_graph_mr(int chunk) {
   CKV(cudaStreamBeginCapture(S->stream, cudaStreamCaptureModeThreadLocal));
   bool ok = true;
   const unsigned long long l0 = S->launches;
-  for (int it = 0; it < chunk && ok; it++) ok = launch_fl_blk_dir<T, NR>(it & 1) && launch_fl_blk_apply<T, NR>(it & 1);
+  for (int it = 0; it < chunk && ok; it++) ok = enqueue_fl_blk_iteration<NR>();
   S->launches = l0;
   cudaError_t e = cudaStreamEndCapture(S->stream, &g);
   if (!ok || e != cudaSuccess) { set_err("block graph capture", cudaGetErrorString(e)); return false; }
@@ -381,8 +366,8 @@ static bool solve_block_minres_device(const bool* has_x0) {
   CKV(cudaMemsetAsync(B->d0, 0, tot * sizeof(T), S->stream));
   CKV(cudaEventRecord(S->ev0, S->stream));
   auto op_k = [&](int k, int fin, bool skip) {
-    return launch_mr_op_buf<T>(slice<T>(B->r, k), slice<T>(B->d1, k), slice<T>(B->q, k), slice<T>(B->s, k),
-                               slice<double>(B->x, k), slice<T>(B->d0, k), fin, skip);
+    return launch_mr_op_buf<T>(slice<T>(B->r, k), nullptr, slice<T>(B->q, k), slice<T>(B->s, k), slice<double>(B->x, k),
+                               slice<T>(B->d0, k), fin, skip);
   };
   for (int k = 0; k < NR; k++) {  // pminres.cu:58-98 per right-hand side
     S->cur_sc = B->sc + k;
@@ -453,7 +438,7 @@ static bool solve_block_minres_device(const bool* has_x0) {
     for (int k = 0; k < NR; k++) any = any || !B->h_sc[k].done;
     if (!any) break;
     CKV(cudaGraphLaunch(B->gexec, S->stream));
-    S->launches += (unsigned long long)chunk * 2;
+    S->launches += (unsigned long long)chunk * 3;
   }
   CKV(cudaEventRecord(S->ev2, S->stream));
   CKV(cudaEventSynchronize(S->ev2));
@@ -545,7 +530,8 @@ static bool solve_block_T(int nr, const double* const* rhs, const double* const*
   bool ok;
   if (S->fluid) {
     if (nr != 3) { set_err("cudapcgB200SolveBlock", "Stokes blocks hold the 3 flow directions"); return false; }
-    ok = solve_block_minres_device<T, 3>(has_x0);
+    if constexpr (sizeof(T) == 8) ok = solve_block_minres_device<T, 3>(has_x0);
+    else { set_err("cudapcgB200SolveBlock", "Stokes models solve in FP64"); return false; }
   } else if (S->nd == 1 && nr == 3) ok = solve_block_device<1, T, 3>(has_x0);
   else if (S->nd == 3 && nr == 6) ok = solve_block_device<3, T, 6>(has_x0);
   else if (S->nd == 3 && nr == 3) ok = solve_block_device<3, T, 3>(has_x0);

@@ -28,7 +28,7 @@
 #include "modal_point.cuh"
 #include "stencil_2d.cuh"
 #include "pore_maps.h"
-#include "stencil_fluid_block.cuh"
+#include "stencil_fluid_mr.cuh"
 #include "loadcase.cuh"
 #include "fields.cuh"
 #include "minres.cuh"
@@ -132,7 +132,8 @@ struct Solver {
   int vec_prec = -1;
   int vec_layout = -1;  // which work vectors ensure_vectors allocated (precision, solver kind)
   void* r = nullptr; void* r2 = nullptr; void* d0 = nullptr; void* d1 = nullptr;
-  void* q = nullptr; void* s = nullptr; void* q2 = nullptr;
+  void* q = nullptr; void* s = nullptr;
+  double* fl_z = nullptr;  // Stokes (P)MINRES: z = M^-1 r as one record per node (stencil_fluid_mr.cuh)
   // FP64 in every mode: the solution, the right-hand side, an operator output and staging
   double* x = nullptr;
   double* b64 = nullptr;
@@ -228,8 +229,9 @@ static void invalidate_graphs() {
 static void free_work_vectors() {
   if (!S) return;
   free_ptr(S->r); free_ptr(S->r2); free_ptr(S->d0); free_ptr(S->d1);
-  free_ptr(S->q); free_ptr(S->s); free_ptr(S->q2);
-  S->r = S->r2 = S->d0 = S->d1 = S->q = S->s = S->q2 = nullptr;
+  free_ptr(S->q); free_ptr(S->s); free_ptr(S->fl_z);
+  S->r = S->r2 = S->d0 = S->d1 = S->q = S->s = nullptr;
+  S->fl_z = nullptr;
   S->vec_prec = -1;
   S->vec_layout = -1;
   if (S->gexec) { cudaGraphExecDestroy(S->gexec); S->gexec = nullptr; S->graph_key = -1; }
@@ -278,7 +280,7 @@ static bool ensure_scratch64(double*& p) {
 //   every solver      x (FP64), r, the direction's two buffers d0 / d1
 //   PCG / MINRES      q = A d
 //   Stokes, MINRES    s (Stokes PCG reads a stored M^-1 r; (P)MINRES keeps A M^-1 r)
-//   MINRES            r2, q2 (the residual's second buffer, the q recursion)
+//   MINRES            thermal, elastic: r2 (the residual's second buffer); Stokes: fl_z
 //   b64 (FP64 right-hand side): kept except for FP64 PCG3, whose r is the only copy of b (as
 //   in the reference's 3-vector solvers, chfem/src/femhmg/cudapcg/solvers/pcg3.cu:28-60)
 // The right-hand side is carried across a change of precision or solver.
@@ -307,11 +309,12 @@ static bool ensure_vectors() {
   std::vector<void**> vs = {&S->r, &S->d0, &S->d1};
   if (!pcg3_solver()) vs.push_back(&S->q);
   if (S->fluid || minres_solver()) vs.push_back(&S->s);
-  if (minres_solver()) { vs.push_back(&S->r2); vs.push_back(&S->q2); }
+  if (minres_solver() && !S->fluid) vs.push_back(&S->r2);
   for (void** v : vs) {
     CKV(dev_malloc(v, n * sizeof(T)));
     CKV(cudaMemsetAsync(*v, 0, n * sizeof(T), S->stream));
   }
+  if (minres_solver() && S->fluid) CKV(dev_malloc(&S->fl_z, (size_t)(S->nV + S->nB) * 4 * 8));
   S->vec_prec = p;
   S->vec_layout = layout;
   if (S->rhs_set && S->b64) {  // re-derive the working right-hand side from its FP64 copy
@@ -321,8 +324,8 @@ static bool ensure_vectors() {
   if (!want_b64 && S->b64) { CKV(cudaStreamSynchronize(S->stream)); free_ptr(S->b64); S->b64 = nullptr; }
   if (p == CHFEM_B200_MIXED && !ensure_scratch64(S->y64)) return false;  // residual replacement
   if (getenv("CHFEM_B200_TRACE"))
-    fprintf(stderr, "[vectors] precision %d layout 0x%x: r %d r2 %d d0 %d d1 %d q %d s %d q2 %d | x %d b64 %d y64 %d x64 %d\n", p, layout,
-            !!S->r, !!S->r2, !!S->d0, !!S->d1, !!S->q, !!S->s, !!S->q2, !!S->x, !!S->b64, !!S->y64, !!S->x64);
+    fprintf(stderr, "[vectors] precision %d layout 0x%x: r %d r2 %d d0 %d d1 %d q %d s %d z %d | x %d b64 %d y64 %d x64 %d\n", p, layout,
+            !!S->r, !!S->r2, !!S->d0, !!S->d1, !!S->q, !!S->s, !!S->fl_z, !!S->x, !!S->b64, !!S->y64, !!S->x64);
   return true;
 }
 
@@ -454,10 +457,7 @@ static bool ensure_K() {
   if (md_applies() && !ensure_md<T>()) return false;
   if (asm_applies() && !ensure_tab<T>()) return false;
   if ((S->d_sdf || S->dim2) && !ensure_invd()) return false;
-  if (S->fluid) {
-    if (sizeof(T) == 8) CKV(cudaMemcpyToSymbol(c_flK64, kt.data(), kt.size() * sizeof(double)));
-    else CKV(cudaMemcpyToSymbol(c_flK32, kt.data(), kt.size() * sizeof(float)));
-  }
+  if (S->fluid && sizeof(T) == 8) CKV(cudaMemcpyToSymbol(c_flK64, kt.data(), kt.size() * sizeof(double)));
   return true;
 }
 
@@ -537,21 +537,26 @@ static bool launch_md(const T* in0, const T* in1, T* vout, T* y, double* x, cons
 template <typename T>
 static bool launch_apply(const T* in0, const T* in1, T* vout, T* y, bool fuse, int finish, bool skip_if_done) {
   if (S->fluid) {
-    FlArgs<T> a;
-    a.v = in0; a.vd = in1; a.vout = vout; a.y = y; a.x = nullptr; a.d = nullptr;
-    a.dof_of_node = S->d_dof_of_node; a.node_of_dof = S->d_node_of_dof; a.bkeys = S->d_bkeys;
-    a.R = S->R; a.C = S->C; a.L = S->L; a.nV = S->nV; a.nB = S->nB;
-    a.sc = S->cur_sc; a.finish = finish; a.skip_if_done = skip_if_done;
-    a.cfg = MrCfg{S->tol, 0, S->resnorm, S->precond, 0};
-    const int g = pw_grid(S->nV + S->nB);
-    if (!ensure_reduction(g)) return false;
-    a.rc = redctl(g);
-    if (S->fdim == 2) {
-      if (fuse) k_fl_apply<T, TE_PCG, 2><<<g, FL_NT, 0, S->stream>>>(a);
-      else k_fl_apply<T, TE_PLAIN, 2><<<g, FL_NT, 0, S->stream>>>(a);
+    if constexpr (sizeof(T) == 8) {  // Stokes models are FP64 in every precision mode
+      FlArgs<T> a;
+      a.v = in0; a.vd = in1; a.vout = vout; a.y = y;
+      a.dof_of_node = S->d_dof_of_node; a.node_of_dof = S->d_node_of_dof; a.bkeys = S->d_bkeys;
+      a.R = S->R; a.C = S->C; a.L = S->L; a.nV = S->nV; a.nB = S->nB;
+      a.sc = S->cur_sc; a.finish = finish; a.skip_if_done = skip_if_done;
+      a.cfg = MrCfg{S->tol, 0, S->resnorm, S->precond, 0};
+      const int g = pw_grid(S->nV + S->nB);
+      if (!ensure_reduction(g)) return false;
+      a.rc = redctl(g);
+      if (S->fdim == 2) {
+        if (fuse) k_fl_apply<T, TE_PCG, 2><<<g, FL_NT, 0, S->stream>>>(a);
+        else k_fl_apply<T, TE_PLAIN, 2><<<g, FL_NT, 0, S->stream>>>(a);
+      } else {
+        if (fuse) k_fl_apply<T, TE_PCG><<<g, FL_NT, 0, S->stream>>>(a);
+        else k_fl_apply<T, TE_PLAIN><<<g, FL_NT, 0, S->stream>>>(a);
+      }
     } else {
-      if (fuse) k_fl_apply<T, TE_PCG><<<g, FL_NT, 0, S->stream>>>(a);
-      else k_fl_apply<T, TE_PLAIN><<<g, FL_NT, 0, S->stream>>>(a);
+      set_err("operator pass", "Stokes models solve in FP64");
+      return false;
     }
   } else if (S->dim2) {
     const int nb = d2_ctas();
@@ -619,11 +624,16 @@ template <typename T, int MODE>
 static bool launch_point(double* x, T* d, T* r, const T* q, T* s, const T* dold) {
   const SolveCfg cfg = solvecfg();
   if (S->fluid) {
-    const int g = pw_grid(S->nV + S->nB);
-    if (!ensure_reduction(g)) return false;
-    FlPw<T> a{x, d, r, q, s, dold, S->d_bkeys, S->nV, S->nB, S->cur_sc, redctl(g), cfg};
-    if (S->fdim == 2) k_fl_point<T, MODE, 2><<<g, PW_NT, 0, S->stream>>>(a);
-    else k_fl_point<T, MODE><<<g, PW_NT, 0, S->stream>>>(a);
+    if constexpr (sizeof(T) == 8) {
+      const int g = pw_grid(S->nV + S->nB);
+      if (!ensure_reduction(g)) return false;
+      FlPw<T> a{x, d, r, q, s, dold, S->d_bkeys, S->nV, S->nB, S->cur_sc, redctl(g), cfg};
+      if (S->fdim == 2) k_fl_point<T, MODE, 2><<<g, PW_NT, 0, S->stream>>>(a);
+      else k_fl_point<T, MODE><<<g, PW_NT, 0, S->stream>>>(a);
+    } else {
+      set_err("pointwise pass", "Stokes models solve in FP64");
+      return false;
+    }
   } else {
     const int g = pw_grid(S->N);
     if (!ensure_reduction(g)) return false;
@@ -862,7 +872,7 @@ static bool run_chunks(bool minres) {
       if (trace) fprintf(stderr, "[single] residual replacement at %d\n", S->h_sc->iteration);
     }
     CKV(cudaGraphLaunch(S->gexec, S->stream));
-    S->launches += (unsigned long long)chunk * 2;
+    S->launches += (unsigned long long)chunk * (minres && S->fluid ? 3 : 2);
   }
   return true;
 }
@@ -1511,6 +1521,20 @@ static bool set_fluid_diag() {
     dg.border[k] = (sum != 0.0) ? 1.0 / sum : 0.0;
   }
   CKV(cudaMemcpyToSymbol(c_fldiag, &dg, sizeof(FlDiag)));
+  // rows of a pore node summed by neighbour (stencil_fluid_mr.cuh), [K G; G^T -Stab]
+  double A[27 * 16] = {0.0};
+  for (int e = 0; e < NE; e++)
+    for (int b = 0; b < NE; b++) {
+      const int o = (drow(b) - drow(e) + 1) + 3 * (dcol(b) - dcol(e) + 1) + (D == 3 ? 9 * (dlay(b) - dlay(e) + 1) : 0);
+      double* blk = A + (size_t)o * (D + 1) * (D + 1);
+      for (int c = 0; c < D; c++) {
+        for (int m = 0; m < D; m++) blk[c * (D + 1) + m] += K[(D * e + c) * ED + D * b + m];
+        blk[c * (D + 1) + D] += K[(D * e + c) * ED + PC + b];
+        blk[D * (D + 1) + c] += K[(PC + e) * ED + D * b + c];
+      }
+      blk[D * (D + 1) + D] -= K[(PC + e) * ED + PC + b];
+    }
+  CKV(cudaMemcpyToSymbol(c_flA, A, sizeof(A)));
   return true;
 }
 
@@ -1678,7 +1702,7 @@ extern "C" {
 template <typename T>
 static double time_kernel_T(int which, unsigned reps) {
   if (!ensure_vectors<T>() || !ensure_K<T>()) return -1.0;
-  if (!S->q || ((which == 3 || which == 4) && !S->r2)) { set_err("cudapcgB200TimeKernel", "kernel not used by the selected solver"); return -1.0; }
+  if (!S->q || ((which == 3 || which == 4) && !S->r2 && !S->fl_z)) { set_err("cudapcgB200TimeKernel", "kernel not used by the selected solver"); return -1.0; }
   if (!ensure_reduction(needed_blocks())) return -1.0;
   // each repetition resets the scalars (so no pass exits early) and brackets only the launch
   float total = 0.f;
@@ -1738,8 +1762,9 @@ unsigned long long cudapcgB200DeviceBytes(void) {
     b += 16ull * n + 8ull * (S->xa_cap + S->hist_cap);
   } else {
     const unsigned long long es = S->vec_prec == CHFEM_B200_FP64 ? 8 : 4;
-    const void* work[] = {S->r, S->r2, S->d0, S->d1, S->q, S->s, S->q2};
+    const void* work[] = {S->r, S->r2, S->d0, S->d1, S->q, S->s};
     for (const void* v : work) b += v ? es * n : 0;
+    b += S->fl_z ? 32ull * (S->nV + S->nB) : 0;
     const double* v64[] = {S->x, S->b64, S->y64, S->x64};
     for (const double* v : v64) b += v ? 8ull * n : 0;
   }
@@ -1747,6 +1772,7 @@ unsigned long long cudapcgB200DeviceBytes(void) {
     const unsigned long long es = B->prec == CHFEM_B200_FP64 ? 8 : 4, tot = (unsigned long long)B->nr * B->n;
     const void* work[] = {B->r, B->s, B->d0, B->d1, B->q};
     for (const void* v : work) b += v ? es * tot : 0;
+    b += B->z ? 32ull * B->nr * (S->nV + S->nB) : 0;
     b += (B->x ? 8ull * tot : 0) + (B->b64 ? 8ull * tot : 0);
   }
   if (S->fluid) b += 4ull * S->N + 4ull * (S->nV + S->nB) + S->nB;

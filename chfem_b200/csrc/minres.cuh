@@ -2,7 +2,7 @@
 // chfem calls MINRES / PMINRES (chfem/src/femhmg/cudapcg/solvers/pminres.cu:163-170,
 // minres.cu:174-181):  z = M^-1 r;  d = z + b d;  q = s + b q;  a = delta / (q . M^-1 q).
 // The other half of the iteration (x += a d, r -= a q, s = A M^-1 r, delta, stopping test)
-// is the TE_MR / fluid MR form of the operator kernels.
+// is the TE_MR form of the operator kernels; the Stokes passes are in stencil_fluid_mr.cuh.
 //
 // Difference from the reference, by design: the reference keeps r in place, turning it into
 // M^-1 r and back with the Jacobi inverse (pminres.cu:172-176); for thermal and elastic
@@ -12,7 +12,6 @@
 #pragma once
 #include "common.cuh"
 #include "stencil_te.cuh"
-#include "stencil_fluid.cuh"
 
 namespace chfem {
 
@@ -56,46 +55,6 @@ __global__ void __launch_bounds__(PW_NT) k_te_mr_dir(MrDirTe<ND, T> a) {
       const T qn = fma(b, a.q[j], a.s[j]);
       a.q[j] = qn;
       sum += (double)qn * (double)(qn * inv[c]);
-    }
-  }
-  const double vals[1] = {sum};
-  const bool ismax[1] = {false};
-  double out[1];
-  if (grid_reduce<PW_NT, 1>(vals, ismax, a.rc, blockIdx.x, out, sred) && threadIdx.x == 0) {
-    a.sc->red[5] = out[0];
-    a.sc->alpha = a.sc->delta / out[0];
-  }
-}
-
-template <typename T>
-struct MrDirFl {
-  T* d; T* q; const T* r; const T* s;
-  const uint8_t* bkeys; long nV, nB;
-  DevScalars* sc; RedCtl rc; int precond;
-};
-
-template <typename T, int DIM = 3>
-__global__ void __launch_bounds__(PW_NT) k_fl_mr_dir(MrDirFl<T> a) {
-  __shared__ double sred[PW_NT / 32];
-  __shared__ double sbd[256];  // interface-node inverse diagonals by fluid key
-  if (a.sc->done) return;
-  for (int i = threadIdx.x; i < 256; i += PW_NT) sbd[i] = c_fldiag.border[i];
-  __syncthreads();
-  const T b = T(a.sc->beta);
-  const long nV = a.nV, nT = a.nV + a.nB;
-  double sum = 0.0;
-  for (long t = blockIdx.x * (long)PW_NT + threadIdx.x; t < nT; t += (long)gridDim.x * PW_NT) {
-    const bool pore = t < nV;
-    const int cnt = pore ? DIM + 1 : 1;
-    for (int k = 0; k < cnt; k++) {
-      const long j = pore ? (k < DIM ? DIM * t + k : DIM * nV + t) : DIM * nV + t;
-      T inv = T(1);
-      if (a.precond) inv = pore ? T(c_fldiag.pore[k]) : T(sbd[a.bkeys[t - nV]]);
-      const T z = a.r[j] * inv;
-      a.d[j] = fma(b, a.d[j], z);
-      const T qn = fma(b, a.q[j], a.s[j]);
-      a.q[j] = qn;
-      sum += (double)qn * (double)(qn * inv);
     }
   }
   const double vals[1] = {sum};

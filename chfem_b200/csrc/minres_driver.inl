@@ -2,7 +2,8 @@
 // Recurrence of chfem/src/femhmg/cudapcg/solvers/pminres.cu:28-247 (and minres.cu:58-260
 // without preconditioner).  Per iteration: the pointwise direction pass finishes alpha, the
 // operator pass updates x and r, applies A to z = M^-1 r and finishes delta, beta and the
-// stopping test.  r alternates between two buffers (read r, write r'), so chunks are even.
+// stopping test.  r alternates between two buffers (read r, write r'), so chunks are even; the
+// Stokes iteration is the three passes of stencil_fluid_mr.cuh, with r in place.
 
 static MrCfg mrcfg() {
   MrCfg cfg;
@@ -11,22 +12,57 @@ static MrCfg mrcfg() {
   return cfg;
 }
 
+// The Stokes passes (stencil_fluid_mr.cuh) on explicit buffers, NR directions n unknowns apart.
+static FlMrArgs fl_mr_args(double* r, double* q, double* s, double* d, double* x, double* z, int fin, bool skip_if_done) {
+  return FlMrArgs{r, q, s, d, x, z, S->d_dof_of_node, S->d_node_of_dof, S->d_bkeys, S->R, S->C, S->L, S->nV, S->nB, S->nvars,
+                  S->cur_sc, RedCtl{}, mrcfg(), fin, skip_if_done};
+}
+template <int NR>
+static bool launch_fl_mr_dir(FlMrArgs a) {
+  const int g = pw_grid(S->nvars);
+  if (!ensure_reduction(g)) return false;
+  a.rc = redctl(g);
+  if (S->fdim == 2) k_fl_mr_dir<NR, 2><<<g, PW_NT, 0, S->stream>>>(a);
+  else k_fl_mr_dir<NR, 3><<<g, PW_NT, 0, S->stream>>>(a);
+  S->launches++;
+  return cudaPeekAtLastError() == cudaSuccess;
+}
+template <int NR>
+static bool launch_fl_mr_upd(const FlMrArgs& a) {
+  const int g = pw_grid(S->nvars);
+  if (S->fdim == 2) k_fl_mr_upd<NR, 2><<<g, PW_NT, 0, S->stream>>>(a);
+  else k_fl_mr_upd<NR, 3><<<g, PW_NT, 0, S->stream>>>(a);
+  S->launches++;
+  return cudaPeekAtLastError() == cudaSuccess;
+}
+template <int NR, int DIM>
+static void launch_fl_mr_apply_dim(const FlMrArgs& a, int g) {
+  if (S->resnorm == CUDAPCG_L2_NORM) k_fl_mr_apply<NR, DIM, false><<<g, FL_NT, 0, S->stream>>>(a);
+  else k_fl_mr_apply<NR, DIM, true><<<g, FL_NT, 0, S->stream>>>(a);
+}
+template <int NR>
+static bool launch_fl_mr_apply(FlMrArgs a) {
+  const int g = pw_grid(S->nV + S->nB);
+  if (!ensure_reduction(g)) return false;
+  a.rc = redctl(g);
+  if (S->fdim == 2) launch_fl_mr_apply_dim<NR, 2>(a, g);
+  else launch_fl_mr_apply_dim<NR, 3>(a, g);
+  S->launches++;
+  return cudaPeekAtLastError() == cudaSuccess;
+}
+
 // Operator pass of (P)MINRES on explicit buffers: r' = r - alpha q into rout, s = A M^-1 r',
 // x += alpha d, with the scalars of S->cur_sc.
 template <typename T>
 static bool launch_mr_op_buf(const T* rin, T* rout, const T* q, T* s, double* x, const T* d, int fin, bool skip_if_done) {
   const MrCfg cfg = mrcfg();
   if (S->fluid) {
-    FlArgs<T> a;
-    a.v = rin; a.vd = q; a.vout = rout; a.y = s; a.x = x; a.d = d;
-    a.dof_of_node = S->d_dof_of_node; a.node_of_dof = S->d_node_of_dof; a.bkeys = S->d_bkeys;
-    a.R = S->R; a.C = S->C; a.L = S->L; a.nV = S->nV; a.nB = S->nB;
-    a.sc = S->cur_sc; a.finish = fin; a.skip_if_done = skip_if_done; a.cfg = cfg;
-    const int g = pw_grid(S->nV + S->nB);
-    if (!ensure_reduction(g)) return false;
-    a.rc = redctl(g);
-    if (S->fdim == 2) k_fl_apply<T, TE_MR, 2><<<g, FL_NT, 0, S->stream>>>(a);
-    else k_fl_apply<T, TE_MR><<<g, FL_NT, 0, S->stream>>>(a);
+    if constexpr (sizeof(T) == 8) {  // r is updated in place (rout unused)
+      if (!launch_fl_mr_upd<1>(fl_mr_args((T*)rin, (T*)q, s, (T*)d, x, S->fl_z, fin, skip_if_done))) return false;
+      return launch_fl_mr_apply<1>(fl_mr_args((T*)rin, (T*)q, s, (T*)d, x, S->fl_z, fin, skip_if_done));
+    }
+    set_err("operator pass", "Stokes models solve in FP64");
+    return false;
   } else if (S->dim2) {
     const int nb = d2_ctas();
     if (!ensure_reduction(nb)) return false;
@@ -90,11 +126,9 @@ static bool launch_mr_op(const T* rin, T* rout, int fin, bool skip_if_done) {
 template <typename T>
 static bool launch_mr_dir(const T* rcur) {
   if (S->fluid) {
-    const int g = pw_grid(S->nV + S->nB);
-    if (!ensure_reduction(g)) return false;
-    MrDirFl<T> a{(T*)S->d0, (T*)S->q, rcur, (const T*)S->s, S->d_bkeys, S->nV, S->nB, S->cur_sc, redctl(g), S->precond};
-    if (S->fdim == 2) k_fl_mr_dir<T, 2><<<g, PW_NT, 0, S->stream>>>(a);
-    else k_fl_mr_dir<T><<<g, PW_NT, 0, S->stream>>>(a);
+    if constexpr (sizeof(T) == 8) return launch_fl_mr_dir<1>(fl_mr_args((T*)rcur, (T*)S->q, (T*)S->s, (T*)S->d0, S->x, S->fl_z, FIN_ALPHA, true));
+    set_err("direction pass", "Stokes models solve in FP64");
+    return false;
   } else {
     const int g = pw_grid(S->N);
     if (!ensure_reduction(g)) return false;
@@ -115,7 +149,8 @@ static bool launch_mr_dir(const T* rcur) {
 
 template <typename T>
 static bool enqueue_minres_iteration(int parity) {
-  const T* rcur = (const T*)(parity ? S->r2 : S->r);
+  // thermal / elastic: the residual alternates between two buffers (Stokes updates it in place)
+  const T* rcur = (const T*)(parity && !S->fluid ? S->r2 : S->r);
   T* rnext = (T*)(parity ? S->r : S->r2);
   return launch_mr_dir<T>(rcur) && launch_mr_op<T>(rcur, rnext, FIN_MR_STEP, true);
 }

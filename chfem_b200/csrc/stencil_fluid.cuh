@@ -23,12 +23,10 @@ constexpr int FL_NT = 256;
 
 template <typename T>
 struct FlArgs {
-  const T* v;          // PLAIN: field | PCG: s | MR: r
-  const T* vd;         // PCG: d_old | MR: q
-  T* vout;             // PCG: formed direction | MR: updated residual r'
+  const T* v;          // PLAIN: field | PCG: s
+  const T* vd;         // PCG: d_old
+  T* vout;             // PCG: formed direction
   T* y;
-  double* x;           // MR: x += alpha d (FP64 in every precision mode)
-  const T* d;          // MR
   const uint32_t* dof_of_node;   // periodic2DOF_map
   const uint32_t* node_of_dof;   // DOF2periodic_map
   const uint8_t* bkeys;          // fluid keys of interface nodes
@@ -41,12 +39,11 @@ struct FlArgs {
   MrCfg cfg;
 };
 
+// Stokes models solve in FP64 in every precision mode (cudapcgB200SetPrecision)
 __constant__ double c_flK64[1024];
-__constant__ float c_flK32[1024];
 
 template <typename T> __device__ __forceinline__ T flK(int i);
 template <> __device__ __forceinline__ double flK<double>(int i) { return c_flK64[i]; }
-template <> __device__ __forceinline__ float flK<float>(int i) { return c_flK32[i]; }
 
 // Jacobi inverse diagonal of a row set: pore rows have fixed values (all 8 voxels fluid);
 // interface rows depend on their fluid key.  Tabulated on the host (256 keys).
@@ -59,10 +56,9 @@ __constant__ FlDiag c_fldiag;
 // Value of the operator's input at DOF `dof` (component comp: 0..DIM-1 velocity, DIM pressure),
 // formed per MODE.  `off` is the vector offset of that entry.
 template <typename T, int MODE>
-__device__ __forceinline__ T fl_in(const FlArgs<T>& a, size_t off, T beta, T alpha, T inv) {
+__device__ __forceinline__ T fl_in(const FlArgs<T>& a, size_t off, T beta) {
   T v = a.v[off];
   if (MODE == TE_PCG) v = fma(beta, a.vd[off], v);
-  if (MODE == TE_MR) v = fma(-alpha, a.vd[off], v) * inv;
   return v;
 }
 
@@ -75,20 +71,11 @@ __global__ void __launch_bounds__(FL_NT) k_fl_apply(FlArgs<T> a) {
   constexpr int NE = 1 << DIM, ED = (DIM + 1) * NE, PC = DIM * NE, NO = DIM == 3 ? 27 : 9;
   constexpr unsigned FULL = (1u << NE) - 1u;
   __shared__ double sred[FL_NT / 32];
-  __shared__ T sbd[256];  // interface-node inverse diagonals by fluid key (per-thread keys: shared, not constant, memory)
   if (a.skip_if_done && a.sc->done) return;
-  for (int i = threadIdx.x; i < 256; i += FL_NT) sbd[i] = T(c_fldiag.border[i]);
-  __syncthreads();
   const long nV = a.nV, nT = a.nV + a.nB;
   const int R = a.R, C = a.C, L = a.L;
   const T beta = (MODE == TE_PCG) ? T(a.sc->beta) : T(0);
-  const T alpha = (MODE == TE_MR && mr_steps(a.finish)) ? T(a.sc->alpha) : T(0);
-  const bool pre = a.cfg.precond != 0;
-  T ivv[DIM];
-#pragma unroll
-  for (int k = 0; k < DIM; k++) ivv[k] = pre ? T(c_fldiag.pore[k]) : T(1);
-  const T ivp = pre ? T(c_fldiag.pore[DIM]) : T(1);
-  double acc = 0.0, acc_rz = 0.0, mr = 0.0, md = 0.0, mx = 0.0;
+  double acc = 0.0;
   for (long t = blockIdx.x * (long)FL_NT + threadIdx.x; t < nT; t += (long)gridDim.x * FL_NT) {
     const uint32_t node = a.node_of_dof[t];
     const int r = (int)(node % (uint32_t)R), c = (int)((node / (uint32_t)R) % (uint32_t)C), l = (int)(node / ((uint32_t)R * (uint32_t)C));
@@ -119,11 +106,9 @@ __global__ void __launch_bounds__(FL_NT) k_fl_apply(FlArgs<T> a) {
       const bool vel = dof < (uint32_t)nV;
       if (vel) {
 #pragma unroll
-        for (int k = 0; k < DIM; k++) vv[k] = fl_in<T, MODE>(a, DIM * (size_t)dof + k, beta, alpha, ivv[k]);
+        for (int k = 0; k < DIM; k++) vv[k] = fl_in<T, MODE>(a, DIM * (size_t)dof + k, beta);
       }
-      T ip = ivp;
-      if (MODE == TE_MR && pre && !vel) ip = sbd[a.bkeys[dof - (uint32_t)nV]];
-      const T vp = fl_in<T, MODE>(a, DIM * (size_t)nV + dof, beta, alpha, ip);
+      const T vp = fl_in<T, MODE>(a, DIM * (size_t)nV + dof, beta);
 #pragma unroll
       for (int e = 0; e < NE; e++) {
 #pragma unroll
@@ -146,7 +131,7 @@ __global__ void __launch_bounds__(FL_NT) k_fl_apply(FlArgs<T> a) {
         }
       }
     }
-    // own rows: formed input (dot), ping-pong outputs, MR updates
+    // own rows: formed input (dot) and outputs
     const int cnt = pore ? DIM + 1 : 1;
     T outv[DIM + 1];
     size_t offs[DIM + 1];
@@ -157,41 +142,19 @@ __global__ void __launch_bounds__(FL_NT) k_fl_apply(FlArgs<T> a) {
     if (!pore) { outv[0] = op; offs[0] = DIM * (size_t)nV + t; }
     for (int k = 0; k < cnt; k++) {
       const size_t j = offs[k];
-      T iv = T(1);
-      if (MODE == TE_MR && pre) iv = pore ? (k == DIM ? ivp : ivv[k < DIM ? k : 0]) : sbd[fk];
-      const T v = fl_in<T, MODE>(a, j, beta, alpha, iv);
+      const T v = fl_in<T, MODE>(a, j, beta);
       a.y[j] = outv[k];
       if (MODE == TE_PCG) a.vout[j] = v;
-      if (MODE == TE_MR) {
-        const T rn = fma(-alpha, a.vd[j], a.v[j]);
-        a.vout[j] = rn;
-        const T dv = a.d[j];
-        const double xv = fma((double)alpha, (double)dv, a.x[j]);
-        a.x[j] = xv;
-        acc_rz += (double)rn * (double)v;
-        mr = fmax(mr, fabs((double)rn));
-        if ((long)j < a.cfg.nhmg) { md = fmax(md, fabs((double)dv)); mx = fmax(mx, fabs((double)xv)); }
-      }
       acc += (double)v * (double)outv[k];
     }
   }
   if (a.finish == 0) return;
-  if (MODE == TE_MR) {
-    const double vals[5] = {acc, acc_rz, mr, md, mx};
-    const bool ismax[5] = {false, false, true, true, true};
-    double out[5];
-    if (grid_reduce<FL_NT, 5>(vals, ismax, a.rc, blockIdx.x, out, sred) && threadIdx.x == 0) {
-      for (int k = 0; k < 5; k++) a.sc->red[k] = out[k];
-      mr_finish(a.finish, out, a.sc, a.cfg);
-    }
-  } else {
-    const double vals[1] = {acc};
-    const bool ismax[1] = {false};
-    double out[1];
-    if (grid_reduce<FL_NT, 1>(vals, ismax, a.rc, blockIdx.x, out, sred) && threadIdx.x == 0) {
-      a.sc->red[0] = out[0];
-      if (a.finish == FIN_ALPHA) a.sc->alpha = a.sc->delta / out[0];
-    }
+  const double vals[1] = {acc};
+  const bool ismax[1] = {false};
+  double out[1];
+  if (grid_reduce<FL_NT, 1>(vals, ismax, a.rc, blockIdx.x, out, sred) && threadIdx.x == 0) {
+    a.sc->red[0] = out[0];
+    if (a.finish == FIN_ALPHA) a.sc->alpha = a.sc->delta / out[0];
   }
 }
 
