@@ -739,15 +739,17 @@ static bool enqueue_pcg3_iteration(int parity) {
          launch_te_mode<T, TE_UPD>(dnew, nullptr, (T*)S->r, S->x, FIN_STORE);
 }
 
-// The pointwise PCG pass of models whose operator runs in voxel modes (modal_point.cuh), on nr
+// The pointwise PCG pass of models whose operator runs in voxel modes and of 2D models
+// (modal_point.cuh), on nr
 // right-hand sides with the scalar records sc.
 template <typename T>
 static bool launch_md_point(int nr, double* x, const T* d, const T* dold, T* r, const T* q, DevScalars* sc, int parity) {
   const int nb = md_point_ctas(S->nvars, num_sms());
   if (!ensure_reduction(nb)) return false;
-  const MdPw<T> a{x, d, dold, r, q, S->d_keys, mddev<T>(), S->d_invd, S->nmat, S->nvars, sc, redctl(nb), solvecfg()};
+  const MdPw<T> a{x, d, dold, r, q, S->d_keys, S->dim2 ? nullptr : mddev<T>(), S->d_invd, S->nmat, S->nvars, sc, redctl(nb), solvecfg()};
   const bool norms = S->resnorm != CUDAPCG_L2_NORM;
-  const cudaError_t e = S->nd == 1 ? md_point_launch<1, T>(nr, a, parity, norms, nb, S->stream) : md_point_launch<3, T>(nr, a, parity, norms, nb, S->stream);
+  // 2D models read the precomputed diagonal per unknown, whatever their unknowns per node
+  const cudaError_t e = S->nd == 1 || S->dim2 ? md_point_launch<1, T>(nr, a, parity, norms, nb, S->stream) : md_point_launch<3, T>(nr, a, parity, norms, nb, S->stream);
   S->launches++;
   if (e != cudaSuccess) { set_err("pointwise pass", cudaGetErrorString(e)); return false; }
   return true;
@@ -758,7 +760,7 @@ static bool enqueue_pcg_iteration(int parity) {
   T* dold = (T*)(parity ? S->d1 : S->d0);
   T* dnew = (T*)(parity ? S->d0 : S->d1);
   if (!launch_apply<T>(pcg_dir_in<T>(), dold, dnew, (T*)S->q, true, FIN_ALPHA, true)) return false;
-  if (md_applies()) return launch_md_point<T>(1, S->x, dnew, dold, (T*)S->r, (const T*)S->q, S->cur_sc, parity);
+  if (md_applies() || S->dim2) return launch_md_point<T>(1, S->x, dnew, dold, (T*)S->r, (const T*)S->q, S->cur_sc, parity);
   return launch_point<T, PW_PCG>(S->x, dnew, (T*)S->r, (const T*)S->q, s_or_null<T>(), nullptr);
 }
 
@@ -1716,7 +1718,7 @@ static double time_kernel_T(int which, unsigned reps) {
       case 0: ok = launch_apply<T>((const T*)S->d0, nullptr, nullptr, (T*)S->q, false, FIN_NONE, false); break;
       case 1: ok = launch_apply<T>(pcg_dir_in<T>(), (const T*)S->d0, (T*)S->d1, (T*)S->q, true, FIN_ALPHA, false); break;
       case 2:
-        ok = md_applies() ? launch_md_point<T>(1, S->x, (const T*)S->d0, (const T*)S->d1, (T*)S->r, (const T*)S->q, S->d_sc, 1)
+        ok = md_applies() || S->dim2 ? launch_md_point<T>(1, S->x, (const T*)S->d0, (const T*)S->d1, (T*)S->r, (const T*)S->q, S->d_sc, 1)
                           : launch_point<T, PW_PCG>(S->x, (T*)S->d1, (T*)S->r, (const T*)S->q, s_or_null<T>(), nullptr);
         break;
       case 3: ok = launch_mr_op<T>((const T*)S->r, (T*)S->r2, FIN_MR_STEP, false); break;

@@ -1,5 +1,5 @@
 // modal_point.cuh -- the pointwise PCG pass of models whose operator passes run in voxel modes
-// (stencil_modal.cuh), for one right-hand side or a block of NR: r -= alpha q, delta = r . M^-1 r,
+// (stencil_modal.cuh) and of 2D models, for one right-hand side or a block of NR: r -= alpha q, delta = r . M^-1 r,
 // the stopping test, and x += alpha d.
 //
 // The solution is updated every second iteration.  d alternates between two buffers, so after an
@@ -25,7 +25,7 @@ struct MdPw {
   double* x; const T* d; const T* dold; T* r; const T* q;  // [NR][n]
   const uint16_t* keys;
   const T* tab;        // the table of the voxel modes: inverse diagonal by material counts
-  const double* invd;  // scalar density field: the inverse diagonal per unknown
+  const double* invd;  // scalar density field, 2D models: the inverse diagonal per unknown (keys, tab unused)
   int nmat;
   long n;
   DevScalars* sc;      // [NR]
@@ -83,7 +83,8 @@ __global__ void __launch_bounds__(MP_NT) k_md_point(MdPw<T> a) {
   if (all) return;
   const int tid = threadIdx.x;
   const bool pre = a.cfg.precond != 0, two = a.nmat <= 2;
-  for (int i = tid; i < (two ? 9 : MD_NCOUNT); i += MP_NT) sTab[i] = pre ? a.tab[i] : T(1);
+  if (pre && !a.invd)
+    for (int i = tid; i < (two ? 9 : MD_NCOUNT); i += MP_NT) sTab[i] = a.tab[i];
   __syncthreads();
   double vals[NV * NR];
 #pragma unroll
@@ -92,7 +93,10 @@ __global__ void __launch_bounds__(MP_NT) k_md_point(MdPw<T> a) {
   auto chunk = [&](long j0, auto width) {
     constexpr int W = decltype(width)::value;
     T inv[W];
-    if (pre && a.invd) {
+    if (!pre) {
+#pragma unroll
+      for (int i = 0; i < W; i++) inv[i] = T(1);
+    } else if (a.invd) {
 #pragma unroll
       for (int i = 0; i < W; i++) inv[i] = T(a.invd[j0 + i]);
     } else if constexpr (ND == 1) {

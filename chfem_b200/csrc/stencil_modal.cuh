@@ -269,7 +269,11 @@ __global__ void __launch_bounds__(MD_NT, MINB) k_modal_apply(MdArgs<ND, typename
   T* sTab = reinterpret_cast<T*>(smem_raw);
   V* sP = reinterpret_cast<V*>(sTab + MD_TAB);  // [4][PPW] formed input
   V* sC = sP + 4 * PPW;                         // [2][4][CW] corner forces
-  for (int i = tid; i < MD_WORDS; i += NT) sTab[i] = (pre || i >= MD_MAT) ? ma.tab[i] : T(1);
+  const int counts = two ? 9 : MD_NCOUNT;  // the entries that the keys' counts can index, then the materials
+  for (int i = tid; i < counts + 8; i += NT) {
+    const int j = i < counts ? i : MD_MAT + i - counts;
+    sTab[j] = (pre || j >= MD_MAT) ? ma.tab[j] : T(1);
+  }
   const DevScalars* sc0 = a.sc + (BLK ? k0 : 0);
   V beta{}, alpha{};
   if constexpr (MODE == TE_PCG || MODE == TE_DIRDOT) {
