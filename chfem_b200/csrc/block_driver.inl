@@ -62,34 +62,17 @@ static bool blk_prepare() {
   return true;
 }
 
-// tile of the FP32 elastic assembled operator: CHFEM_B200_ASM_TILE = "8x1", "6x2", "8x2", "4x2"
-// (columns x layers per thread), "6x1r" or "7x1r" (one layer per thread, 4-slot plane ring)
-static int asm_tile_choice() {
-  static int choice = -1;
-  if (choice < 0) {
-    const char* e = getenv("CHFEM_B200_ASM_TILE");
-    choice = ASM_TILE_8x1;
-    if (e && !strcmp(e, "6x2")) choice = ASM_TILE_6x2;
-    if (e && !strcmp(e, "8x2")) choice = ASM_TILE_8x2;
-    if (e && !strcmp(e, "4x2")) choice = ASM_TILE_4x2;
-    if (e && !strcmp(e, "6x1r")) choice = ASM_TILE_6x1_RING4;
-    if (e && !strcmp(e, "7x1r")) choice = ASM_TILE_7x1_RING4;
-  }
-  return choice;
-}
-
 // The assembled-stencil block operator pass (stencil_asm.cuh, launched from asm_apply.cu), on
 // the NR right-hand sides from k0 on (dold / dnew: the direction buffers of right-hand side 0).
 template <int ND, typename T, int NR>
 static bool launch_asm_block(T* dold, T* dnew, int precond, int k0 = 0) {
-  const int tile = asm_tile_choice();
-  const int nb = asm_block_ctas<ND, T, NR>(S->R, S->C, S->L, num_sms(), tile);
+  const int nb = asm_block_ctas<ND, T, NR>(S->R, S->C, S->L, num_sms());
   if (nb < 1) { set_err("assembled block operator", "launch configuration"); return false; }
   if (!ensure_reduction(nb)) return false;
   const size_t off = (size_t)k0 * S->nvars;
   BlkArgs<ND, T> a{(const T*)B->r + off, dold + off, dnew + off, (T*)B->q + off, S->d_keys, Kdev<T>(), S->nmat, S->R, S->C, S->L,
                    S->nvars, B->sc + k0, redctl(nb), precond};
-  const cudaError_t e = asm_block_launch<ND, T, NR>(a, tabdev<T>(), nb, tile, S->stream);
+  const cudaError_t e = asm_block_launch<ND, T, NR>(a, tabdev<T>(), nb, S->stream);
   S->launches++;
   if (e != cudaSuccess) { set_err("assembled block operator", cudaGetErrorString(e)); return false; }
   return true;
