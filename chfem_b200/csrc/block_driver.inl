@@ -8,7 +8,7 @@ struct BlockState {
   long n = 0;
   void *r = nullptr, *s = nullptr, *d0 = nullptr, *d1 = nullptr, *q = nullptr;  // [nr][n], work precision
   double *x = nullptr, *b64 = nullptr;                                          // [nr][n], FP64
-  double* z = nullptr;        // Stokes: the records of z = M^-1 r, [nV + nB][nr][4]
+  double* z = nullptr;        // Stokes: the records of z = M^-1 r, [nodes or fluid nodes][nr][4]
   DevScalars* sc = nullptr;   // [nr]
   DevScalars* h_sc = nullptr; // pinned [nr]
   double* d_mom = nullptr;    // load-case moments [BLK_MAX][8] + CB staging
@@ -43,7 +43,7 @@ static bool block_alloc(int nr) {
   // operator pass); Stokes (P)MINRES: r, d, q, s = A M^-1 r and z
   std::vector<void**> vs = {&B->r, &B->d0, &B->q};
   vs.push_back(S->fluid ? &B->s : &B->d1);
-  if (S->fluid) CKV(dev_malloc(&B->z, (size_t)(S->nV + S->nB) * nr * 4 * 8));
+  if (S->fluid) CKV(dev_malloc(&B->z, fl_record_bytes(nr)));
   for (void** v : vs) { CKV(dev_malloc(v, tot * sizeof(T))); CKV(cudaMemset(*v, 0, tot * sizeof(T))); }
   CKV(dev_malloc(&B->x, tot * 8));
   CKV(dev_malloc(&B->b64, tot * 8));
@@ -313,7 +313,7 @@ static bool solve_block_device(const bool* has_x0) {
 // q = A d B->q, s = A M^-1 r B->s, z = M^-1 r B->z; r is updated in place.
 template <int NR>
 static bool enqueue_fl_blk_iteration() {
-  FlMrArgs a = fl_mr_args((double*)B->r, (double*)B->q, (double*)B->s, (double*)B->d0, B->x, B->z, FIN_MR_STEP, true);
+  FlMrArgs a = fl_mr_args(B->nr, (double*)B->r, (double*)B->q, (double*)B->s, (double*)B->d0, B->x, B->z, FIN_MR_STEP, true);
   a.sc = B->sc;
   return launch_fl_mr_dir<NR>(a) && launch_fl_mr_upd<NR>(a) && launch_fl_mr_apply<NR>(a);
 }

@@ -276,6 +276,8 @@ static bool ensure_scratch64(double*& p) {
   return true;
 }
 
+static size_t fl_record_bytes(int nr);
+
 // Work vectors for precision T, as many as the selected solver reads:
 //   every solver      x (FP64), r, the direction's two buffers d0 / d1
 //   PCG / MINRES      q = A d
@@ -314,7 +316,7 @@ static bool ensure_vectors() {
     CKV(dev_malloc(v, n * sizeof(T)));
     CKV(cudaMemsetAsync(*v, 0, n * sizeof(T), S->stream));
   }
-  if (minres_solver() && S->fluid) CKV(dev_malloc(&S->fl_z, (size_t)(S->nV + S->nB) * 4 * 8));
+  if (minres_solver() && S->fluid) CKV(dev_malloc(&S->fl_z, fl_record_bytes(1)));
   S->vec_prec = p;
   S->vec_layout = layout;
   if (S->rhs_set && S->b64) {  // re-derive the working right-hand side from its FP64 copy
@@ -1523,6 +1525,7 @@ static bool set_fluid_diag() {
     dg.border[k] = (sum != 0.0) ? 1.0 / sum : 0.0;
   }
   CKV(cudaMemcpyToSymbol(c_fldiag, &dg, sizeof(FlDiag)));
+  CKV(cudaMemcpyToSymbol(d_flborder, dg.border, sizeof(dg.border)));
   // rows of a pore node summed by neighbour (stencil_fluid_mr.cuh), [K G; G^T -Stab]
   double A[27 * 16] = {0.0};
   for (int e = 0; e < NE; e++)
@@ -1766,7 +1769,7 @@ unsigned long long cudapcgB200DeviceBytes(void) {
     const unsigned long long es = S->vec_prec == CHFEM_B200_FP64 ? 8 : 4;
     const void* work[] = {S->r, S->r2, S->d0, S->d1, S->q, S->s};
     for (const void* v : work) b += v ? es * n : 0;
-    b += S->fl_z ? 32ull * (S->nV + S->nB) : 0;
+    b += S->fl_z ? fl_record_bytes(1) : 0;
     const double* v64[] = {S->x, S->b64, S->y64, S->x64};
     for (const double* v : v64) b += v ? 8ull * n : 0;
   }
@@ -1774,7 +1777,7 @@ unsigned long long cudapcgB200DeviceBytes(void) {
     const unsigned long long es = B->prec == CHFEM_B200_FP64 ? 8 : 4, tot = (unsigned long long)B->nr * B->n;
     const void* work[] = {B->r, B->s, B->d0, B->d1, B->q};
     for (const void* v : work) b += v ? es * tot : 0;
-    b += B->z ? 32ull * B->nr * (S->nV + S->nB) : 0;
+    b += B->z ? fl_record_bytes(B->nr) : 0;
     b += (B->x ? 8ull * tot : 0) + (B->b64 ? 8ull * tot : 0);
   }
   if (S->fluid) b += 4ull * S->N + 4ull * (S->nV + S->nB) + S->nB;

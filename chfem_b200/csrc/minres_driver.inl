@@ -12,9 +12,16 @@ static MrCfg mrcfg() {
   return cfg;
 }
 
-// The Stokes passes (stencil_fluid_mr.cuh) on explicit buffers, NR directions n unknowns apart.
-static FlMrArgs fl_mr_args(double* r, double* q, double* s, double* d, double* x, double* z, int fin, bool skip_if_done) {
-  return FlMrArgs{r, q, s, d, x, z, S->d_dof_of_node, S->d_node_of_dof, S->d_bkeys, S->R, S->C, S->L, S->nV, S->nB, S->nvars,
+// Whether the Stokes records of nr directions are kept per grid node (stencil_fluid_mr.cuh): 8 %
+// faster than per fluid node at 96^3 and porosity 0.35, for 32 N nr bytes instead of 32 (nV + nB) nr.
+// Not where the grid holds more than four nodes per fluid node or its records exceed 16 GiB, so
+// that a model that fills the device memory needs no more of it.
+static bool fl_by_node(int nr) { return S->N <= 4l * (S->nV + S->nB) && 32l * S->N * nr <= 16l << 30; }
+static size_t fl_record_bytes(int nr) { return 32ul * nr * std::max(fl_by_node(nr) ? S->N : S->nV + S->nB, 1l); }
+
+// The Stokes passes (stencil_fluid_mr.cuh) on explicit buffers, nr directions n unknowns apart.
+static FlMrArgs fl_mr_args(int nr, double* r, double* q, double* s, double* d, double* x, double* z, int fin, bool skip_if_done) {
+  return FlMrArgs{r, q, s, d, x, z, S->d_node_of_dof, S->d_bkeys, fl_by_node(nr) ? nullptr : S->d_dof_of_node, S->R, S->C, S->L, S->nV, S->nB, S->nvars,
                   S->cur_sc, RedCtl{}, mrcfg(), fin, skip_if_done};
 }
 template <int NR>
@@ -35,18 +42,19 @@ static bool launch_fl_mr_upd(const FlMrArgs& a) {
   S->launches++;
   return cudaPeekAtLastError() == cudaSuccess;
 }
-template <int NR, int DIM>
+template <int NR, int DIM, bool GRID>
 static void launch_fl_mr_apply_dim(const FlMrArgs& a, int g) {
-  if (S->resnorm == CUDAPCG_L2_NORM) k_fl_mr_apply<NR, DIM, false><<<g, FL_NT, 0, S->stream>>>(a);
-  else k_fl_mr_apply<NR, DIM, true><<<g, FL_NT, 0, S->stream>>>(a);
+  if (S->resnorm == CUDAPCG_L2_NORM) k_fl_mr_apply<NR, DIM, false, GRID><<<g, FL_NT, 0, S->stream>>>(a);
+  else k_fl_mr_apply<NR, DIM, true, GRID><<<g, FL_NT, 0, S->stream>>>(a);
 }
 template <int NR>
 static bool launch_fl_mr_apply(FlMrArgs a) {
   const int g = pw_grid(S->nV + S->nB);
   if (!ensure_reduction(g)) return false;
   a.rc = redctl(g);
-  if (S->fdim == 2) launch_fl_mr_apply_dim<NR, 2>(a, g);
-  else launch_fl_mr_apply_dim<NR, 3>(a, g);
+  const bool grid = !a.dof_of_node;
+  if (S->fdim == 2) grid ? launch_fl_mr_apply_dim<NR, 2, true>(a, g) : launch_fl_mr_apply_dim<NR, 2, false>(a, g);
+  else grid ? launch_fl_mr_apply_dim<NR, 3, true>(a, g) : launch_fl_mr_apply_dim<NR, 3, false>(a, g);
   S->launches++;
   return cudaPeekAtLastError() == cudaSuccess;
 }
@@ -58,8 +66,8 @@ static bool launch_mr_op_buf(const T* rin, T* rout, const T* q, T* s, double* x,
   const MrCfg cfg = mrcfg();
   if (S->fluid) {
     if constexpr (sizeof(T) == 8) {  // r is updated in place (rout unused)
-      if (!launch_fl_mr_upd<1>(fl_mr_args((T*)rin, (T*)q, s, (T*)d, x, S->fl_z, fin, skip_if_done))) return false;
-      return launch_fl_mr_apply<1>(fl_mr_args((T*)rin, (T*)q, s, (T*)d, x, S->fl_z, fin, skip_if_done));
+      if (!launch_fl_mr_upd<1>(fl_mr_args(1, (T*)rin, (T*)q, s, (T*)d, x, S->fl_z, fin, skip_if_done))) return false;
+      return launch_fl_mr_apply<1>(fl_mr_args(1, (T*)rin, (T*)q, s, (T*)d, x, S->fl_z, fin, skip_if_done));
     }
     set_err("operator pass", "Stokes models solve in FP64");
     return false;
@@ -126,7 +134,7 @@ static bool launch_mr_op(const T* rin, T* rout, int fin, bool skip_if_done) {
 template <typename T>
 static bool launch_mr_dir(const T* rcur) {
   if (S->fluid) {
-    if constexpr (sizeof(T) == 8) return launch_fl_mr_dir<1>(fl_mr_args((T*)rcur, (T*)S->q, (T*)S->s, (T*)S->d0, S->x, S->fl_z, FIN_ALPHA, true));
+    if constexpr (sizeof(T) == 8) return launch_fl_mr_dir<1>(fl_mr_args(1, (T*)rcur, (T*)S->q, (T*)S->s, (T*)S->d0, S->x, S->fl_z, FIN_ALPHA, true));
     set_err("direction pass", "Stokes models solve in FP64");
     return false;
   } else {

@@ -5,14 +5,18 @@
 // An iteration is three passes:
 //   k_fl_mr_dir    d = M^-1 r + beta d, q = s + beta q, and alpha = delta / (q . M^-1 q);
 //   k_fl_mr_upd    r -= alpha q, x += alpha d, and z = M^-1 r, stored as one record of 4 doubles
-//                  per DOF-numbered node and direction -- DIM velocities and the pressure; an
-//                  interface node's velocities are 0 (no slip);
+//                  per grid node and direction -- DIM velocities and the pressure; an interface
+//                  node's velocities are 0 (no slip), solid nodes' records are never touched;
+//                  where the grid is large against its fluid nodes (fl_by_node), per fluid node;
 //   k_fl_mr_apply  s = A z, delta = z . s, r . z, the max-norms where the stopping test reads
 //                  them, and the finisher (mr_finish).
-// The gather over a node's 27 neighbours then loads one 32-byte record and one DOF number per
-// neighbour.  (Forming z = M^-1 (r - alpha q) in the gather, which saves the middle pass, took 8
-// loads of 8 bytes and 4 multiply-adds per neighbour and bound the operator by its loads: 0.30 ms
-// at 128^3 against the figures at k_fl_mr_apply.)  r is no neighbour input of any pass and is
+// The gather over a node's 27 neighbours then loads one 32-byte record each, at constant offsets
+// from the node's own (periodic wraps aside): no DOF number on the way, so the loads do not wait
+// on one another.  It is bound by their latency.  Measured at 96^3, porosity 0.35, one direction:
+// forming z = M^-1 (r - alpha q) in the gather (8 loads of 8 bytes and 4 multiply-adds per
+// neighbour) 139 us an iteration, records by DOF number 76 us, by grid node 70 us.  The records of a
+// grid cost 32 bytes per node and direction of memory, and no more traffic: a fluid node's
+// neighbours within its fluid voxels are fluid nodes.  r is no neighbour input of any pass and is
 // updated in place.
 //
 // The row of a pore node (all its voxels fluid) is summed by neighbour once per model on the
@@ -30,8 +34,9 @@ __constant__ double c_flA[27 * 16];
 
 struct FlMrArgs {
   double* r; double* q; double* s; double* d; double* x;  // [NR][n]
-  double* z;                                              // [nV + nB][NR][4]
-  const uint32_t* dof_of_node; const uint32_t* node_of_dof; const uint8_t* bkeys;
+  double* z;                                              // [nodes or fluid nodes][NR][4]
+  const uint32_t* node_of_dof; const uint8_t* bkeys;
+  const uint32_t* dof_of_node;  // records per fluid node: their numbers; per grid node: null
   int R, C, L;
   long nV, nB, n;   // n: unknowns per direction
   DevScalars* sc;   // [NR]
@@ -48,6 +53,13 @@ __device__ __forceinline__ double fl_mr_inv(long j, long nV, const uint8_t* bkey
   return j < (DIM + 1) * nV ? c_fldiag.pore[DIM] : sbd[bkeys[j - (DIM + 1) * nV]];
 }
 
+// the interface diagonals in shared memory, from an array (constant memory serialises lanes that
+// read different entries)
+__device__ double d_flborder[256];
+__device__ __forceinline__ void fl_mr_table(double* sbd) {
+  for (int i = threadIdx.x; i < 256; i += PW_NT) sbd[i] = d_flborder[i];
+}
+
 // whether a pass has nothing to do; done[k]: direction k has stopped (its vectors stay)
 template <int NR>
 __device__ __forceinline__ bool fl_mr_done(const FlMrArgs& a, bool (&done)[NR]) {
@@ -59,25 +71,41 @@ __device__ __forceinline__ bool fl_mr_done(const FlMrArgs& a, bool (&done)[NR]) 
 
 template <int NR, int DIM>
 __global__ void __launch_bounds__(PW_NT) k_fl_mr_dir(FlMrArgs a) {
+  constexpr int U = NR == 1 ? 4 : 2;  // unknowns per thread and step, their loads issued together
   __shared__ double sred[PW_NT / 32];
   __shared__ double sbd[256];
+  fl_mr_table(sbd);
   bool done[NR];
   if (fl_mr_done<NR>(a, done)) return;
-  for (int i = threadIdx.x; i < 256; i += PW_NT) sbd[i] = c_fldiag.border[i];
-  __syncthreads();
   double beta[NR], sum[NR];
 #pragma unroll
   for (int k = 0; k < NR; k++) { beta[k] = a.sc[k].beta; sum[k] = 0.0; }
-  for (long j = blockIdx.x * (long)PW_NT + threadIdx.x; j < a.n; j += (long)gridDim.x * PW_NT) {
-    const double inv = fl_mr_inv<DIM>(j, a.nV, a.bkeys, sbd, a.cfg.precond != 0);
+  __syncthreads();
+  const long step = (long)gridDim.x * PW_NT;
+  for (long j0 = blockIdx.x * (long)PW_NT + threadIdx.x; j0 < a.n; j0 += U * step) {
+    double inv[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) inv[u] = j0 + u * step < a.n ? fl_mr_inv<DIM>(j0 + u * step, a.nV, a.bkeys, sbd, a.cfg.precond != 0) : 0.0;
 #pragma unroll
     for (int k = 0; k < NR; k++) {
       if (NR > 1 && done[k]) continue;
-      const long i = k * a.n + j;
-      a.d[i] = fma(beta[k], a.d[i], a.r[i] * inv);
-      const double qn = fma(beta[k], a.q[i], a.s[i]);
-      a.q[i] = qn;
-      sum[k] += qn * (qn * inv);
+      double r[U], s[U], d[U], q[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const long i = k * a.n + j0 + u * step;
+        const bool in = j0 + u * step < a.n;
+        r[u] = in ? a.r[i] : 0.0; s[u] = in ? a.s[i] : 0.0; d[u] = in ? a.d[i] : 0.0; q[u] = in ? a.q[i] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const long i = k * a.n + j0 + u * step;
+        const double qn = fma(beta[k], q[u], s[u]);
+        if (j0 + u * step < a.n) {
+          a.d[i] = fma(beta[k], d[u], r[u] * inv[u]);
+          a.q[i] = qn;
+          sum[k] += qn * (qn * inv[u]);
+        }
+      }
     }
   }
   const bool ismax[NR] = {};
@@ -92,36 +120,55 @@ __global__ void __launch_bounds__(PW_NT) k_fl_mr_dir(FlMrArgs a) {
 // finish codes without a step (the initial residual, an initial guess) take alpha = 0
 template <int NR, int DIM>
 __global__ void __launch_bounds__(PW_NT) k_fl_mr_upd(FlMrArgs a) {
+  constexpr int U = NR == 1 ? 4 : 2;
   __shared__ double sbd[256];
+  fl_mr_table(sbd);
   bool done[NR];
   if (fl_mr_done<NR>(a, done)) return;
-  for (int i = threadIdx.x; i < 256; i += PW_NT) sbd[i] = c_fldiag.border[i];
-  __syncthreads();
-  const bool step = a.finish == FIN_MR_STEP;
+  const bool move = a.finish == FIN_MR_STEP;
   double alpha[NR];
 #pragma unroll
-  for (int k = 0; k < NR; k++) alpha[k] = step ? a.sc[k].alpha : 0.0;
-  const long nVD = DIM * a.nV;
-  for (long j = blockIdx.x * (long)PW_NT + threadIdx.x; j < a.n; j += (long)gridDim.x * PW_NT) {
-    const double inv = fl_mr_inv<DIM>(j, a.nV, a.bkeys, sbd, a.cfg.precond != 0);
-    const bool vel = j < nVD;
-    const long dof = vel ? j / DIM : j - nVD;
-    const int comp = vel ? (int)(j - dof * DIM) : DIM;
+  for (int k = 0; k < NR; k++) alpha[k] = move ? a.sc[k].alpha : 0.0;
+  __syncthreads();
+  const long nVD = DIM * a.nV, step = (long)gridDim.x * PW_NT;
+  for (long j0 = blockIdx.x * (long)PW_NT + threadIdx.x; j0 < a.n; j0 += U * step) {
+    double inv[U];
+    long rec[U];  // the unknown's place in its node's records (direction 0)
+    bool edge[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const long j = j0 + u * step;
+      const bool in = j < a.n, vel = j < nVD;
+      const long dof = vel ? j / DIM : j - nVD;
+      inv[u] = in ? fl_mr_inv<DIM>(j, a.nV, a.bkeys, sbd, a.cfg.precond != 0) : 0.0;
+      rec[u] = in ? (a.dof_of_node ? dof : (long)a.node_of_dof[dof]) * (4 * NR) + (vel ? j - dof * DIM : DIM) : 0;
+      edge[u] = !vel && dof >= a.nV;
+    }
 #pragma unroll
     for (int k = 0; k < NR; k++) {
       if (NR > 1 && done[k]) continue;
-      const long i = k * a.n + j;
-      double rn = a.r[i];
-      if (step) {
-        rn = fma(-alpha[k], a.q[i], rn);
-        a.r[i] = rn;
-        a.x[i] = fma(alpha[k], a.d[i], a.x[i]);
-      }
-      double* zr = a.z + (dof * NR + k) * 4;
-      zr[comp] = rn * inv;
-      if (!vel && dof >= a.nV) {  // interface node: no velocity
+      double r[U], q[U], d[U], x[U];
 #pragma unroll
-        for (int c = 0; c < DIM; c++) zr[c] = 0.0;
+      for (int u = 0; u < U; u++) {
+        const long i = k * a.n + j0 + u * step;
+        const bool in = j0 + u * step < a.n, m = in && move;
+        r[u] = in ? a.r[i] : 0.0; q[u] = m ? a.q[i] : 0.0; d[u] = m ? a.d[i] : 0.0; x[u] = m ? a.x[i] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (j0 + u * step >= a.n) continue;
+        const long i = k * a.n + j0 + u * step;
+        const double rn = fma(-alpha[k], q[u], r[u]);
+        if (move) {
+          a.r[i] = rn;
+          a.x[i] = fma(alpha[k], d[u], x[u]);
+        }
+        double* z = a.z + rec[u] + 4 * k;
+        *z = rn * inv[u];
+        if (edge[u]) {  // interface node: no velocity
+#pragma unroll
+          for (int c = 1; c <= DIM; c++) z[-c] = 0.0;
+        }
       }
     }
   }
@@ -146,8 +193,8 @@ __host__ __device__ constexpr unsigned fl_mr_emask(int o) {
   return m;
 }
 
-// MAXN: the stopping test reads max-norms (infinity / error norm).
-template <int NR, int DIM, bool MAXN>
+// MAXN: the stopping test reads max-norms (infinity / error norm).  GRID: records per grid node.
+template <int NR, int DIM, bool MAXN, bool GRID>
 __global__ void __launch_bounds__(FL_NT, NR == 1 ? 3 : 2) k_fl_mr_apply(FlMrArgs a) {
   constexpr int NE = 1 << DIM, ED = (DIM + 1) * NE, PC = DIM * NE, NO = DIM == 3 ? 27 : 9, D1 = DIM + 1;
   constexpr int NV = MAXN ? 5 : 2;
@@ -175,11 +222,12 @@ __global__ void __launch_bounds__(FL_NT, NR == 1 ? 3 : 2) k_fl_mr_apply(FlMrArgs
     if (pore) {
 #pragma unroll
       for (int o = 0; o < NO; o++) {
-        const long dof = o == NO / 2 ? t : (long)a.dof_of_node[rr[o % 3] + cc[(o / 3) % 3] + ll[DIM == 3 ? o / 9 : 1]];
+        size_t nb = rr[o % 3] + cc[(o / 3) % 3] + ll[DIM == 3 ? o / 9 : 1];
+        if constexpr (!GRID) nb = a.dof_of_node[nb];
 #pragma unroll
         for (int k = 0; k < NR; k++) {
           double v[4];
-          fl_mr_rec(a.z + (dof * NR + k) * 4, v);
+          fl_mr_rec(a.z + (nb * NR + k) * 4, v);
 #pragma unroll
           for (int i = 0; i < D1; i++)
 #pragma unroll
@@ -204,11 +252,12 @@ __global__ void __launch_bounds__(FL_NT, NR == 1 ? 3 : 2) k_fl_mr_apply(FlMrArgs
               for (int m = 0; m < DIM; m++) g[m] += c_flK64[(PC + e) * ED + DIM * b + m];
               g[DIM] -= c_flK64[(PC + e) * ED + PC + b];
             }
-        const long dof = o == NO / 2 ? t : (long)a.dof_of_node[rr[o % 3] + cc[(o / 3) % 3] + ll[DIM == 3 ? o / 9 : 1]];
+        size_t nb = rr[o % 3] + cc[(o / 3) % 3] + ll[DIM == 3 ? o / 9 : 1];
+        if constexpr (!GRID) nb = a.dof_of_node[nb];
 #pragma unroll
         for (int k = 0; k < NR; k++) {
           double v[4];
-          fl_mr_rec(a.z + (dof * NR + k) * 4, v);
+          fl_mr_rec(a.z + (nb * NR + k) * 4, v);
 #pragma unroll
           for (int m = 0; m < D1; m++) out[k][DIM] = fma(g[m], v[m], out[k][DIM]);
         }
@@ -218,7 +267,7 @@ __global__ void __launch_bounds__(FL_NT, NR == 1 ? 3 : 2) k_fl_mr_apply(FlMrArgs
     for (int k = 0; k < NR; k++) {
       if (NR > 1 && done[k]) continue;
       double own[4];
-      fl_mr_rec(a.z + (t * NR + k) * 4, own);
+      fl_mr_rec(a.z + ((size_t)(GRID ? node : t) * NR + k) * 4, own);
 #pragma unroll
       for (int i = 0; i < D1; i++) {
         if (i < DIM && !pore) continue;
