@@ -75,16 +75,17 @@ __global__ void __launch_bounds__(MP_NT) k_md_point(MdPw<T> a) {
   bool all = true;
 #pragma unroll
   for (int k = 0; k < NR; k++) {
+    const double al = a.sc[k].alpha;  // read beside done, not after it
     done[k] = a.sc[k].done;
     xa[k] = XM == 1 ? a.sc[k].xa : 0.0;
-    alpha[k] = done[k] ? 0.0 : a.sc[k].alpha;
+    alpha[k] = done[k] ? 0.0 : al;
     all = all && done[k] && xa[k] == 0.0;
   }
-  if (all) return;
   const int tid = threadIdx.x;
   const bool pre = a.cfg.precond != 0, two = a.nmat <= 2;
   if (pre && !a.invd)
     for (int i = tid; i < (two ? 9 : MD_NCOUNT); i += MP_NT) sTab[i] = a.tab[i];
+  if (all) return;
   __syncthreads();
   double vals[NV * NR];
 #pragma unroll

@@ -206,26 +206,33 @@ inline size_t md_smem_bytes() {
 // How the work line of a pass -- (column tile, layer) units -- is cut for P CTAs: one run each
 // where that costs fewer layers (a run restages 3), else equal slices of the line (TeWork).
 struct MdWork {
-  TeWork te;
+  int R, C, L, tiles_r, tiles;
   int nc;  // one run per CTA: chunks of layers per tile; 0: slices
   int P, bid;
-  __device__ MdWork(int R, int C, int L, int P_, int bid_) : te(R, C, L, MD_TC), nc(0), P(P_), bid(bid_) {
-    const long per = P / te.tiles;
+  __device__ MdWork(int R_, int C_, int L_, int P_, int bid_) : R(R_), C(C_), L(L_), nc(0), P(P_), bid(bid_) {
+    tiles_r = (R + TE_TR - 1) / TE_TR;
+    tiles = tiles_r * ((C + MD_TC - 1) / MD_TC);
+    const int per = P / tiles;
     if (per >= 1) {
-      const int n = (int)min((long)L, per);
-      if ((L + n - 1) / n + 3 <= (te.W + P - 1) / P + 6) nc = n;
+      const int n = min(L, per);
+      if ((float)((L + n - 1) / n + 3) <= (float)tiles * (float)L / (float)P + 6.f) nc = n;
     }
-    if (!nc) te.share(P);
   }
-  __device__ long begin() const { return nc ? 0 : (long)bid * te.W / P; }
-  __device__ long end() const { return nc ? (bid < nc * te.tiles ? 1 : 0) : ((long)bid + 1) * te.W / P; }
+  __device__ TeWork slices() const {
+    TeWork w(R, C, L, MD_TC);
+    w.share(P);
+    return w;
+  }
+  __device__ long begin() const { return nc ? 0 : (long)bid * ((long)tiles * L) / P; }
+  __device__ long end() const { return nc ? (bid < nc * tiles ? 1 : 0) : ((long)bid + 1) * ((long)tiles * L) / P; }
   __device__ void run(long w, long w_end, int& r0, int& c0, int& l0, int& l1) const {
-    if (!nc) { te.run(w, w_end, r0, c0, l0, l1); return; }
-    const int c = bid / (int)te.tiles, t = bid - c * (int)te.tiles;
-    l0 = (int)((long)c * te.L / nc);
-    l1 = (int)((long)(c + 1) * te.L / nc);
-    r0 = (t % te.tiles_r) * TE_TR;
-    c0 = (t / te.tiles_r) * MD_TC;
+    if (!nc) { slices().run(w, w_end, r0, c0, l0, l1); return; }
+    const int c = bid / tiles, t = bid - c * tiles;
+    const int q = L / nc, rem = L - q * nc;  // the first rem chunks hold one layer more
+    l0 = c * q + min(c, rem);
+    l1 = l0 + q + (c < rem ? 1 : 0);
+    r0 = (t % tiles_r) * TE_TR;
+    c0 = (t / tiles_r) * MD_TC;
   }
   __device__ long step(int l0, int l1) const { return nc ? 1 : l1 - l0; }
 };
@@ -246,6 +253,15 @@ __global__ void __launch_bounds__(MD_NT, MINB) k_modal_apply(MdArgs<ND, typename
   __shared__ double sred[NT / 32];
   const auto& a = ma.te;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const bool pre = a.cfg.precond != 0, two = a.nmat <= 2;
+  T* sTab = reinterpret_cast<T*>(smem_raw);
+  auto table = [&]() {  // filled while the scalar records are on their way
+    const int counts = two ? 9 : MD_NCOUNT;  // the entries that the keys' counts can index, then the materials
+    for (int i = tid; i < counts + 8; i += NT) {
+      const int j = i < counts ? i : MD_MAT + i - counts;
+      sTab[j] = (pre || j >= MD_MAT) ? ma.tab[j] : T(1);
+    }
+  };
   // the group of right-hand sides and this CTA's share of its work line
   int k0 = 0, P = gridDim.x, bid = blockIdx.x;
   bool idle = false;
@@ -253,6 +269,7 @@ __global__ void __launch_bounds__(MD_NT, MINB) k_modal_apply(MdArgs<ND, typename
   if constexpr (BLK) {
     live = 0u;
     for (int k = 0; k < ma.nr; k++) live |= a.sc[k].done ? 0u : 1u << k;
+    table();
     if (!live) return;
     int ng = 0;
     for (int g = 0; g < ma.nr / W; g++) ng += (live >> (g * W)) & ((1u << W) - 1u) ? 1 : 0;
@@ -263,17 +280,12 @@ __global__ void __launch_bounds__(MD_NT, MINB) k_modal_apply(MdArgs<ND, typename
     for (int g = 0; g < ma.nr / W; g++)
       if ((live >> (g * W)) & ((1u << W) - 1u)) { if (ga == 0) k0 = g * W; ga--; }
   } else {
-    if (a.skip_if_done && a.sc->done) return;
+    const int done = a.skip_if_done ? a.sc->done : 0;
+    table();
+    if (done) return;
   }
-  const bool pre = a.cfg.precond != 0, two = a.nmat <= 2;
-  T* sTab = reinterpret_cast<T*>(smem_raw);
   V* sP = reinterpret_cast<V*>(sTab + MD_TAB);  // [4][PPW] formed input
   V* sC = sP + 4 * PPW;                         // [2][4][CW] corner forces
-  const int counts = two ? 9 : MD_NCOUNT;  // the entries that the keys' counts can index, then the materials
-  for (int i = tid; i < counts + 8; i += NT) {
-    const int j = i < counts ? i : MD_MAT + i - counts;
-    sTab[j] = (pre || j >= MD_MAT) ? ma.tab[j] : T(1);
-  }
   const DevScalars* sc0 = a.sc + (BLK ? k0 : 0);
   V beta{}, alpha{};
   if constexpr (MODE == TE_PCG || MODE == TE_DIRDOT) {
