@@ -28,6 +28,7 @@
 #include "pointwise.cuh"
 #include "stencil_te.cuh"
 #include "stencil_block.cuh"
+#include "stencil_modal.cuh"
 #include "loadcase.cuh"
 
 namespace chfem {
@@ -51,7 +52,7 @@ struct BtSched {
   int n_act;  // active samples
   int pending;  // a load case awaits replacement or a check (mixed precision)
   long W;     // work units (tile, layer) over the active samples
-  long Nn;    // nodes over the active samples
+  long Nn;    // groups of 4 nodes over the active samples
 };
 
 // Everything the batch passes read; device pointers.
@@ -63,12 +64,13 @@ struct BtData {
   const uint16_t* keys;      // [noff[n]]
   const TV* K;               // [n][4][64] dense conductivity matrices (slots past nmat zero)
   const double* K64;         // same in FP64 (replacement operator, right-hand sides)
+  const double* lam;         // [n][4] constants of the voxel modes (k / 16 per material), or null
   DevScalars* sc;            // [n][3]
   BtCtl* ctl;                // [n][3]
   const BtSched* sch;
   const int* act;            // [n] active sample ids
   const long* wpre;          // [n+1] work prefix over active samples
-  const long* npre;          // [n+1] node prefix over active samples
+  const long* npre;          // [n+1] prefix of 4-node groups over active samples
   double* part;              // [(P + n) * 3] partials
   unsigned* ticket;
   int* pending;              // &BtSched::pending: raised by the pointwise finisher, cleared by the replacement pass
@@ -104,6 +106,29 @@ __device__ __forceinline__ int bt_cta_of(long w, long W, int P) {
 // they write no partials)
 __device__ __forceinline__ bool bt_nonempty(int b, long W, int P) { return ((long)(b + 1) * W) / P > ((long)b * W) / P; }
 
+// Jacobi diagonal of the nodes of one sample whose conductivity matrices are isotropic, from its
+// materials' diagonal values (0 past the last): tabulated by the count of material 1 for at most
+// two materials, else summed by the counts and inverted.
+template <typename T>
+struct BtDiag {
+  T d[4], inv9[9];
+  int two;
+};
+template <typename T>
+__device__ __forceinline__ void bt_diag_fill(BtDiag<T>& b, const double* K64, int tid, bool pre) {
+  if (tid < 4) b.d[tid] = pre ? T(K64[64 * tid]) : T(tid == 0 ? 0.125 : 0.0);
+  if (tid < 9) b.inv9[tid] = pre ? T(1.0 / ((8 - tid) * K64[0] + tid * K64[64])) : T(1);
+  if (tid == 0) b.two = !pre || (K64[128] == 0.0 && K64[192] == 0.0);
+}
+template <typename T>
+__device__ __forceinline__ T bt_inv(const BtDiag<T>& b, unsigned key) {
+  const unsigned lo = key & 0x5555u;
+  if (b.two) return b.inv9[__popc(lo)];
+  const unsigned hi = (key >> 1) & 0x5555u;
+  const int n3 = __popc(lo & hi), n1 = __popc(lo) - n3, n2 = __popc(hi) - n3;
+  return T(1) / (T(8 - n1 - n2 - n3) * b.d[0] + T(n1) * b.d[1] + T(n2) * b.d[2] + T(n3) * b.d[3]);
+}
+
 // Active list: samples with a load case still iterating (or pending a check), with prefix
 // sums of their work units and nodes.  One CTA of 1024 threads.
 template <int TC>
@@ -122,7 +147,7 @@ __global__ void __launch_bounds__(1024) k_bt_schedule(int n, const int* dims, co
     if (i < n)
       for (int k = 0; k < BT_NR; k++) on = on || !sc[BT_NR * i + k].done || ctl[BT_NR * i + k].pending != BT_NONE;
     const long w = on ? bt_tiles<TC>(dims, i) * dims[3 * i + 2] : 0;
-    const long nn = on ? bt_nodes(dims, i) : 0;
+    const long nn = on ? (bt_nodes(dims, i) + 3) / 4 : 0;
     sw[tid] = w; sn[tid] = nn; sf[tid] = on ? 1 : 0;
     __syncthreads();
     for (int o = 1; o < 1024; o <<= 1) {  // inclusive scans
@@ -147,6 +172,35 @@ __global__ void __launch_bounds__(1024) k_bt_schedule(int n, const int* dims, co
     wpre[ca] = cw; npre[ca] = cn;
     sch->n_act = ca; sch->W = cw; sch->Nn = cn;
   }
+}
+
+// The last CTA of an operator pass finishes alpha_k = delta_k / (d_k . A d_k) per active sample.
+template <typename TV, int NT>
+__device__ inline void bt_finish_alpha(const BtData<TV>& a, const BtSched& sch, int P, long W) {
+  __shared__ bool s_last;
+  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+  if (tid == 0) {
+    __threadfence();
+    s_last = atomicAdd(a.ticket, 1u) == (unsigned)P - 1u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  for (int ii = tid; ii < sch.n_act; ii += NT) {
+    const int b0 = bt_cta_of(a.wpre[ii], W, P), b1 = bt_cta_of(a.wpre[ii + 1] - 1, W, P);
+    const int ss = a.act[ii];
+#pragma unroll
+    for (int k = 0; k < BT_NR; k++) {
+      DevScalars& sc = a.sc[BT_NR * ss + k];
+      if (sc.done) continue;
+      double sum = 0.0;
+      for (int b = b0; b <= b1; b++)
+        if (bt_nonempty(b, W, P)) sum += __ldcg(a.part + ((long)b + ii) * BT_NR + k);
+      sc.red[0] = sum;
+      sc.alpha = sc.delta / sum;
+    }
+  }
+  if (tid == 0) *a.ticket = 0u;
 }
 
 // Operator pass over the work line.  RES = false: the block PCG pass, v_k = s_k + beta_k d_k
@@ -268,33 +322,174 @@ __global__ void __launch_bounds__(TE_TR * TC) k_bt_apply(BtData<TV> a, const TV*
   }
   if (RES) return;
   if (cur >= 0) flush(cur);
-  // the last CTA finishes alpha_k = delta_k / (d_k . A d_k) per active sample
-  __shared__ bool s_last;
-  if (tid == 0) {
-    __threadfence();
-    s_last = atomicAdd(a.ticket, 1u) == (unsigned)P - 1u;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  for (int ii = tid; ii < sch.n_act; ii += NT) {
-    const int b0 = bt_cta_of(a.wpre[ii], W, P), b1 = bt_cta_of(a.wpre[ii + 1] - 1, W, P);
-    const int ss = a.act[ii];
+  bt_finish_alpha<TV, NT>(a, sch, P, W);
+}
+
+// The same pass in voxel modes (stencil_modal.cuh), for batches whose conductivity matrices are
+// all isotropic: 32 x 8 columns, a thread per node of the haloed plane, the sample's three load
+// cases together (they share the node's key and all index arithmetic).  sv: r, of which M^-1 r is formed
+// here and never stored.  A load case that does not take part is neither read nor written.
+constexpr int BM_CW = MD_PR * (MD_TC + 1);  // one corner's forces of a plane
+template <typename TS>
+inline size_t bt_modal_smem() { return (size_t)BT_NR * (4 * MD_PP + 8 * BM_CW) * sizeof(TS); }
+
+template <typename TV, bool RES>
+__global__ void __launch_bounds__(MD_NT, (RES || sizeof(TV) == 8) ? 1 : 2) k_bt_modal(BtData<TV> a, const TV* sv, const TV* dold, TV* dnew, TV* q,
+                                                                                       const double* x, const double* b64, TV* r) {
+  using TS = std::conditional_t<RES, double, TV>;  // staging / compute type
+  constexpr int NT = MD_NT, PP = MD_PP, PR = MD_PR, CW = BM_CW;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TS* sP = reinterpret_cast<TS*>(smem_raw);  // [4][BT_NR][PP] formed input
+  TS* sC = sP + 4 * BT_NR * PP;              // [2][4][BT_NR][CW] corner forces
+  __shared__ double sred[NT / 32];
+  __shared__ TS sbeta[BT_NR], slam[4];
+  __shared__ BtDiag<TS> sdiag;
+  __shared__ int son[BT_NR];  // load case served by this pass
+  const BtSched sch = *a.sch;
+  if (sch.n_act == 0 || (RES && !sch.pending)) return;
+  const int P = gridDim.x, bid = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  const long W = sch.W, w0 = (long)bid * W / P, w1 = ((long)bid + 1) * W / P;
+  const int vr = tid % PR, vc = tid / PR;
+  const bool point = tid < PP, voxel = vr < PR - 1 && vc < MD_TC + 1;
+  double acc[BT_NR] = {0.0, 0.0, 0.0};
+  int cur = -1, s = 0, R = 1, C = 1, L = 1, tiles_r = 1;
+  long nbase = 0, vbase = 0, Ns = 0;
+  bool on[BT_NR] = {false, false, false};
+  auto flush = [&](int i) {
+    if constexpr (!RES) {
 #pragma unroll
-    for (int k = 0; k < BT_NR; k++) {
-      DevScalars& sc = a.sc[BT_NR * ss + k];
-      if (sc.done) continue;
-      double sum = 0.0;
-      for (int b = b0; b <= b1; b++)
-        if (bt_nonempty(b, W, P)) sum += __ldcg(a.part + ((long)b + ii) * BT_NR + k);
-      sc.red[0] = sum;
-      sc.alpha = sc.delta / sum;
+      for (int k = 0; k < BT_NR; k++) {
+        const double t = block_sum<NT>(acc[k], sred);
+        if (tid == 0) a.part[((long)bid + i) * BT_NR + k] = t;
+        acc[k] = 0.0;
+      }
+    }
+  };
+  int i = (w0 < w1) ? bt_find(a.wpre, sch.n_act, w0) : 0;
+  for (long w = w0; w < w1;) {
+    while (w >= a.wpre[i + 1]) i++;
+    if (i != cur) {
+      if (cur >= 0) flush(cur);
+      cur = i;
+      s = a.act[i];
+      R = a.dims[3 * s]; C = a.dims[3 * s + 1]; L = a.dims[3 * s + 2];
+      tiles_r = (R + TE_TR - 1) / TE_TR;
+      nbase = a.noff[s]; Ns = (long)R * C * L; vbase = BT_NR * nbase;
+      __syncthreads();
+      if (tid < 4) slam[tid] = TS(a.lam[4 * s + tid]);
+      if (!RES) bt_diag_fill<TS>(sdiag, a.K64 + (size_t)s * 256, tid, a.cfg.precond != 0);
+      if (tid < BT_NR) {
+        const DevScalars& scs = a.sc[BT_NR * s + tid];
+        if (RES) son[tid] = a.ctl[BT_NR * s + tid].pending != BT_NONE;
+        else son[tid] = !scs.done;
+        sbeta[tid] = RES ? TS(0) : TS(scs.beta);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < BT_NR; k++) on[k] = son[k];
+    }
+    const long u = w - a.wpre[i];
+    const int tile = (int)(u / L), l0 = (int)(u - (long)tile * L);
+    const int l1 = (int)min((long)L, (long)l0 + (min(w1, a.wpre[i + 1]) - w));
+    w += l1 - l0;
+    if (!(on[0] || on[1] || on[2])) continue;
+    const int r0 = (tile % tiles_r) * TE_TR, c0 = (tile / tiles_r) * MD_TC;
+    const long RC = (long)R * C;
+    const int node = point ? wrap(r0 + vr - 1, R) + wrap(c0 + vc - 1, C) * R : 0;
+    const bool act = wp < MD_TC && c0 + wp < C && r0 + lane < R;
+    const int onode = r0 + lane + (c0 + wp) * R;
+    auto first = [&](int l) { return (long)(l < 0 ? l + L : (l >= L ? l - L : l)) * RC; };
+    TS g0[BT_NR], g1[BT_NR];
+    unsigned gk = 0, vmat = 0;
+    auto load = [&](int l) {
+      if (!point) return;
+      const long j0 = first(l) + node;
+      gk = a.keys[nbase + j0];
+#pragma unroll
+      for (int k = 0; k < BT_NR; k++) {
+        if (!on[k]) continue;
+        const long j = vbase + k * Ns + j0;
+        if (RES) g0[k] = TS(x[j]);
+        else { g0[k] = TS(sv[j]); g1[k] = TS(dold[j]); }
+      }
+    };
+    TS mo[BT_NR][4], fc[BT_NR][1][4];
+#pragma unroll
+    for (int k = 0; k < BT_NR; k++) g0[k] = g1[k] = TS(0);
+    __syncthreads();  // the previous run's reads of the planes are done
+    load(l0 - 1);
+    for (int l = l0 - 1; l <= l1 + 1; l++) {
+      TS v[BT_NR];
+      unsigned vnext = 0;
+      if (l <= l1) {
+        vnext = md_material(gk);
+        const TS inv = RES ? TS(1) : bt_inv<TS>(sdiag, gk);
+#pragma unroll
+        for (int k = 0; k < BT_NR; k++) {
+          v[k] = RES ? g0[k] : TS(fma(sbeta[k], g1[k], inv * g0[k]));
+          if (point) sP[((l & 3) * BT_NR + k) * PP + tid] = v[k];
+        }
+        if (l < l1) load(l + 1);
+      }
+      __syncthreads();
+      if (l <= l1 && voxel) {
+        const TS lam = slam[vmat];
+#pragma unroll
+        for (int k = 0; k < BT_NR; k++) {
+          if (!on[k]) continue;
+          const TS* pl = sP + ((l & 3) * BT_NR + k) * PP + tid;
+          TS nm[1][4];
+          md_plane<TS>(v[k], pl[1], pl[PR], pl[PR + 1], nm[0]);
+          if (l >= l0) {
+            TS ms[1][4], mdif[1][4], fa[1][4];
+            md_layers<TS>(mo[k], nm[0], ms[0], mdif[0]);
+            md_voxel<1, TS, TS>(ms, mdif, lam, lam, fc[k], fa);
+            if (l > l0) {
+              TS* f = sC + ((l & 1) * 4 * BT_NR + k) * CW + tid;
+              TS f00, f10, f01, f11;
+              md_plane_t<TS>(fa[0], f00, f10, f01, f11);
+              f[0] = f00;
+              f[BT_NR * CW] = f10;
+              f[2 * BT_NR * CW] = f01;
+              f[3 * BT_NR * CW] = f11;
+            }
+          } else {
+#pragma unroll
+            for (int m = 0; m < 4; m++) fc[k][0][m] = TS(0);
+          }
+#pragma unroll
+          for (int m = 0; m < 4; m++) mo[k][m] = nm[0][m];
+        }
+      }
+      vmat = vnext;
+      if (l - 2 >= l0 && act) {
+        const long j0 = first(l - 2) + onode;
+#pragma unroll
+        for (int k = 0; k < BT_NR; k++) {
+          if (!on[k]) continue;
+          const TS* f = sC + (((l - 1) & 1) * 4 * BT_NR + k) * CW + wp * PR + lane;
+          const TS out = (f[PR + 1] + f[BT_NR * CW + PR]) + (f[2 * BT_NR * CW + 1] + f[3 * BT_NR * CW]);
+          const long j = vbase + k * Ns + j0;
+          if (RES) {
+            r[j] = TV(b64[j] - (double)out);
+          } else {
+            const TS vv = sP[(((l - 2) & 3) * BT_NR + k) * PP + (wp + 1) * PR + lane + 1];
+            q[j] = TV(out);
+            dnew[j] = TV(vv);
+            acc[k] += (double)vv * (double)out;
+          }
+        }
+      }
     }
   }
-  if (tid == 0) *a.ticket = 0u;
+  if (RES) return;
+  if (cur >= 0) flush(cur);
+  bt_finish_alpha<TV, NT>(a, sch, P, W);
 }
 
 // Pointwise pass over the node line of the active samples.
+// A thread takes 4 nodes of every load case (16-byte accesses where the sample's vectors allow
+// them); sv null: s = M^-1 r is not stored (the modal operator forms it).
 //   PW_INIT: s = M^-1 r, delta0 (zero guess); PW_PCG: x += a d, r -= a q, s = M^-1 r, delta,
 //   stopping test (and, mixed, the replacement / check decisions); PW_REPL: for pending load
 //   cases, s = M^-1 r from the true residual, then the replacement or check finisher.
@@ -302,12 +497,14 @@ template <typename TV, int MODE>
 __global__ void __launch_bounds__(PW_NT) k_bt_point(BtData<TV> a, double* x, const TV* d, TV* r, const TV* q, TV* sv) {
   __shared__ double sred[PW_NT / 32];
   __shared__ TV sD[32];
+  __shared__ BtDiag<TV> sdiag;
   __shared__ double salpha[BT_NR];
   __shared__ int son[BT_NR];
   const BtSched sch = *a.sch;
   if (sch.n_act == 0 || (MODE == PW_REPL && !sch.pending)) return;
   const int P = gridDim.x, bid = blockIdx.x, tid = threadIdx.x;
   const long Nn = sch.Nn, n0 = (long)bid * Nn / P, n1 = ((long)bid + 1) * Nn / P;
+  const bool iso = a.lam != nullptr;
   double acc[BT_NR] = {0.0, 0.0, 0.0};
   int cur = -1;
   auto flush = [&](int i) {
@@ -326,10 +523,14 @@ __global__ void __launch_bounds__(PW_NT) k_bt_point(BtData<TV> a, double* x, con
       cur = i;
       const int s = a.act[i];
       __syncthreads();
-      for (int t = tid; t < 32; t += PW_NT) {
-        const int m = t >> 3, k = t & 7;
-        const TV dv = a.K[(size_t)s * 256 + m * 64 + k * 9];
-        sD[t] = (dv != TV(0)) ? dv : TV(1);
+      if (iso) {
+        bt_diag_fill<TV>(sdiag, a.K64 + (size_t)s * 256, tid, a.cfg.precond != 0);
+      } else {
+        for (int t = tid; t < 32; t += PW_NT) {
+          const int m = t >> 3, k = t & 7;
+          const TV dv = a.K[(size_t)s * 256 + m * 64 + k * 9];
+          sD[t] = (dv != TV(0)) ? dv : TV(1);
+        }
       }
       if (tid < BT_NR) {
         const DevScalars& scs = a.sc[BT_NR * s + tid];
@@ -345,27 +546,66 @@ __global__ void __launch_bounds__(PW_NT) k_bt_point(BtData<TV> a, double* x, con
     const long seg_end = min(n1, a.npre[i + 1]);
     const long loc0 = v0 - a.npre[i];
     const long cnt = seg_end - v0;
+    const bool vec = Ns % 4 == 0 && nbase % 4 == 0;  // every vector of the sample starts on 4 words
     if (son[0] || son[1] || son[2]) {
-      for (long t = tid; t < cnt; t += PW_NT) {
-        const long node = loc0 + t;
-        TV inv[1];
-        if (a.cfg.precond) te_invdiag<1, TV>(sD, a.keys[nbase + node], inv);
-        else inv[0] = TV(1);
+      for (long t = tid; t < cnt; t += PW_NT) {  // 4 nodes of every load case
+        const long node = 4 * (loc0 + t);
+        const int m = (int)min(4L, Ns - node);
+        TV inv[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          const unsigned key = a.keys[nbase + node + min(u, m - 1)];
+          if (iso) {
+            inv[u] = bt_inv<TV>(sdiag, key);
+          } else {
+            TV iv[1] = {TV(1)};
+            if (a.cfg.precond) te_invdiag<1, TV>(sD, key, iv);
+            inv[u] = iv[0];
+          }
+        }
 #pragma unroll
         for (int k = 0; k < BT_NR; k++) {
           if (!son[k]) continue;
           const size_t j = vbase + k * Ns + node;
-          TV rv = r[j];
-          if (MODE == PW_PCG) {
-            const double al = salpha[k];
-            const TV dv = d[j];
-            x[j] = fma(al, (double)dv, x[j]);
-            rv = fma(-TV(al), q[j], rv);
-            r[j] = rv;
+          const double al = salpha[k];
+          TV rv[4], dv[4], qv[4];
+          double xv[4];
+          if (vec) {
+            blk_ld4(r + j, rv);
+            if (MODE == PW_PCG) {
+              blk_ld4(d + j, dv);
+              blk_ld4(q + j, qv);
+              blk_ld4(x + j, xv);
+            }
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              const size_t ju = j + min(u, m - 1);
+              rv[u] = r[ju];
+              if (MODE == PW_PCG) { dv[u] = d[ju]; qv[u] = q[ju]; xv[u] = x[ju]; }
+            }
           }
-          const TV s_ = rv * inv[0];
-          sv[j] = s_;
-          acc[k] += (double)rv * (double)s_;
+          TV sn[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            if (MODE == PW_PCG) {
+              xv[u] = fma(al, (double)dv[u], xv[u]);
+              rv[u] = fma(-TV(al), qv[u], rv[u]);
+            }
+            sn[u] = rv[u] * inv[u];
+            if (u < m) acc[k] += (double)rv[u] * (double)sn[u];
+          }
+          if (vec) {
+            if (MODE == PW_PCG) { blk_st4(x + j, xv); blk_st4(r + j, rv); }
+            if (sv) blk_st4(sv + j, sn);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              if (u >= m) break;
+              if (MODE == PW_PCG) { x[j + u] = xv[u]; r[j + u] = rv[u]; }
+              if (sv) sv[j + u] = sn[u];
+            }
+          }
         }
       }
     }

@@ -85,3 +85,46 @@ def test_batch_many_uneven_samples():
     export_for_chfem(os.path.join(d, "o.raw"), imgs[i], 0, mat_props=props[i], solver_tolerance=1e-8, solver_maxiter=20000)
     Cref, _ = H.run_exec(H.ORACLE_EXEC, os.path.join(d, "o.nf"), os.path.join(d, "o.raw"))
     assert H.rel_to_max(Cb[i], Cref) < 1e-6
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("precondition", [0, 1])
+@pytest.mark.parametrize("sizes", [[((1, 2, 3), 2)], [((1, 1, 1), 1), ((9, 33, 31), 4), ((4, 8, 32), 3), ((33, 7, 5), 2), ((3, 9, 65), 1)]])
+def test_batch_in_voxel_modes_equals_general_pass(tmp_path, sizes, precision, precondition):
+    """One matrix off an isotropic one by 1e-10 sends the whole batch to the passes for any matrices
+    (C ABI): the moments differ by that and by what two solves to 1e-10 differ."""
+    import ctypes
+    from chfem_b200 import _native
+    from tests.test_gpu_parity import build_small, host_arrays
+    models = [host_arrays(*build_small(tmp_path, f"bm{i}", 0, ("img", shp, nmat))) for i, (shp, nmat) in enumerate(sizes)]
+    lib = _native.cudapcg()
+    n = len(models)
+    rng = np.random.default_rng(9)
+    keys = [np.ascontiguousarray(m["keys"]) for m in models]
+    # rows that sum to zero, as every flux average's: the solution's constant is not determined
+    CB = [rng.standard_normal((m["nkeys"], 3, 8)) for m in models]
+    CB = [np.ascontiguousarray(c - c.mean(axis=2, keepdims=True)).reshape(-1) for c in CB]
+    dims = np.array([[m["ny"], m["nx"], m["nz"]] for m in models], np.uint32)
+    nmat = np.array([m["nkeys"] for m in models], np.uint32)
+    # the conductivity matrix of a unit voxel: 1D stiffness along an axis times the other axes' masses
+    at = np.array([(0, 0, 1), (0, 1, 1), (0, 1, 0), (0, 0, 0), (1, 0, 1), (1, 1, 1), (1, 1, 0), (1, 0, 0)])
+    same = at[:, None, :] == at[None, :, :]
+    S, M = np.where(same, 1.0, -1.0), np.where(same, 1 / 3, 1 / 6)
+    Ke = sum(S[..., i] * M[..., (i + 1) % 3] * M[..., (i + 2) % 3] for i in range(3))
+    v = np.array([1.0, -1, 1, -1, 0, 0, 0, 0])
+    out = []
+    for eps in (0.0, 1e-10):
+        K = [np.concatenate([k * Ke.reshape(-1) for k in (1.0, 10.0, 3.0, 0.5)[:m["nkeys"]]]) for m in models]
+        K[0][:64] += eps * np.outer(v, v).reshape(-1)
+        P = lambda arrs: (ctypes.c_void_p * n)(*[a.ctypes.data for a in arrs])
+        moments, its, res = np.zeros(9 * n), np.zeros(3 * n, np.uint32), np.zeros(3 * n)
+        lib.cudapcgB200BatchLastError.restype = ctypes.c_char_p
+        rc = lib.cudapcgB200SolveThermalBatch(
+            ctypes.c_uint(n), dims.ctypes.data_as(ctypes.c_void_p), P(keys), nmat.ctypes.data_as(ctypes.c_void_p), P(K), P(CB),
+            ctypes.c_double(1e-10 if precision == 0 else 1e-7), ctypes.c_uint(5000), precision, precondition,
+            moments.ctypes.data_as(ctypes.c_void_p), its.ctypes.data_as(ctypes.c_void_p), res.ctypes.data_as(ctypes.c_void_p), None)
+        assert rc == 1, lib.cudapcgB200BatchLastError()
+        out.append((moments, its.astype(int)))
+    (m0, i0), (m1, i1) = out
+    assert H.rel_to_max(m0, m1) < (1e-8 if precision == 0 else 1e-4)
+    assert np.abs(i0 - i1).max() <= (1 if precision == 0 else 5), (i0, i1)
