@@ -68,11 +68,22 @@ def chfem():
         lib.chfemB200Run.argtypes = [c.c_void_p, c.c_char_p, c.c_int, c.c_int, c.c_int, c.c_int, c.c_int, c.c_void_p]
         lib.chfemB200Run.restype = c.c_int
         lib.chfemB200SetExportFields.argtypes = [c.c_int]
+        lib.chfemB200ColorHistogram.argtypes = [c.c_void_p, c.c_ulonglong, c.c_void_p]
+        lib.chfemB200ColorHistogram.restype = c.c_int
         lib.chfemB200RunThermalBatch.argtypes = [c.c_uint, c.c_void_p, c.c_double, c.c_uint, c.c_int, c.c_void_p, c.c_void_p,
                                                  c.c_void_p]
         lib.chfemB200RunThermalBatch.restype = c.c_int
         lib._typed = True
     return lib
+
+
+def color_histogram(array):
+    """Voxels of each of the 256 colours of a C-contiguous uint8 array."""
+    counts = (ctypes.c_ulonglong * 256)()
+    lib = chfem()
+    if not lib.chfemB200ColorHistogram(array.ctypes.data, array.size, counts):
+        raise RuntimeError(lib.chfemB200LastError().decode())
+    return counts
 
 
 class BatchStats(ctypes.Structure):

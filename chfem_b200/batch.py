@@ -11,6 +11,7 @@ import ctypes
 import numpy as np
 
 from . import _native
+from .io import _color_histogram
 
 
 def compute_conductivity_batch(arrays, mat_props, solver_tolerance=1e-6, solver_maxiter=10000, precision="fp64",
@@ -38,7 +39,7 @@ def compute_conductivity_batch(arrays, mat_props, solver_tolerance=1e-6, solver_
             raise ValueError("each image must be a 3D (z, y, x) array")
         if not 1 <= len(p) <= 4:
             raise ValueError("1 to 4 materials per image")
-        present = set(np.unique(a).tolist())
+        present = set(np.nonzero(_color_histogram(a))[0].tolist())
         missing = present - set(int(c) for c in p)
         if missing:
             raise ValueError(f"image {s}: colours {sorted(missing)} have no conductivity")

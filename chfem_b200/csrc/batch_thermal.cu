@@ -9,12 +9,14 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/cudapcg_b200.h"
 #include "batch_thermal.cuh"
 #include "loadcase.cuh"
+#include "devpool.h"
 #include "modal_apply.h"
 
 using namespace chfem;
@@ -31,17 +33,63 @@ std::string g_err;
 // tile width chosen per batch signature (sizes histogram, precision)
 std::map<std::string, int> g_tile_cache;
 
+// The stream, its events and the pinned schedule record of a batch serve the next one on the same
+// device (as cudapcgEnd keeps a solver's: their destruction alone cost up to 0.7 s a call).  At
+// most 4 sets are kept, for as many threads; a batch that failed destroys its own.
+struct BtHandles {
+  int dev = -1;
+  cudaStream_t st = nullptr;
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+  BtSched* h_sch = nullptr;
+};
+std::mutex g_idle_mutex;
+std::vector<BtHandles> g_idle;
+bool take_handles(BtHandles& h) {
+  int dev = -1;
+  BT_CK(cudaGetDevice(&dev));
+  {
+    std::lock_guard<std::mutex> lock(g_idle_mutex);
+    for (size_t i = 0; i < g_idle.size(); i++)
+      if (g_idle[i].dev == dev) {
+        h = g_idle[i];
+        g_idle.erase(g_idle.begin() + i);
+        return true;
+      }
+  }
+  h.dev = dev;
+  BT_CK(cudaStreamCreateWithFlags(&h.st, cudaStreamNonBlocking));
+  for (cudaEvent_t& e : h.ev) BT_CK(cudaEventCreate(&e));
+  BT_CK(cudaMallocHost(&h.h_sch, sizeof(BtSched)));
+  return true;
+}
+void give_handles(BtHandles& h, bool keep) {
+  if (keep) {
+    std::lock_guard<std::mutex> lock(g_idle_mutex);
+    if (g_idle.size() < 4) {
+      g_idle.push_back(h);
+      return;
+    }
+  }
+  if (h.h_sch) cudaFreeHost(h.h_sch);
+  for (cudaEvent_t e : h.ev)
+    if (e) cudaEventDestroy(e);
+  if (h.st) cudaStreamDestroy(h.st);
+}
+
+// Device memory of a batch, from the same pool as the solver's.  The batch waits for its stream
+// before the blocks go back.
 struct DevBuf {
   std::vector<void*> ptrs;
   template <typename T>
   bool alloc(T** p, size_t count) {
     void* q = nullptr;
-    if (cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) { g_err = "cudaMalloc failed (batch too large?)"; return false; }
+    pool_keep();
+    if (cudaMallocAsync(&q, std::max<size_t>(count, 1) * sizeof(T), 0) != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) { g_err = "device allocation failed (batch too large?)"; return false; }
     ptrs.push_back(q);
     *p = (T*)q;
     return true;
   }
-  ~DevBuf() { for (void* p : ptrs) cudaFree(p); }
+  ~DevBuf() { for (void* p : ptrs) cudaFreeAsync(p, 0); }
 };
 
 int num_sms() {
@@ -74,7 +122,9 @@ template <typename TV>
 struct Batch {
   Inputs in;
   DevBuf buf;
-  cudaStream_t st = nullptr;
+  BtHandles h;
+  bool complete = false;    // every launch returned: the handles may serve another batch
+  cudaStream_t st = nullptr;  // h.st
   int* d_dims = nullptr;
   long* d_noff = nullptr;
   uint16_t* d_keys = nullptr;
@@ -86,7 +136,6 @@ struct Batch {
   DevScalars* d_sc = nullptr;
   BtCtl* d_ctl = nullptr;
   BtSched* d_sch = nullptr;
-  BtSched* h_sch = nullptr;
   int* d_act = nullptr;
   long *d_wpre = nullptr, *d_npre = nullptr;
   unsigned* d_ticket = nullptr;
@@ -94,8 +143,8 @@ struct Batch {
   unsigned long long launches = 0;
 
   ~Batch() {
-    if (h_sch) cudaFreeHost(h_sch);
-    if (st) cudaStreamDestroy(st);
+    if (st) complete = cudaStreamSynchronize(st) == cudaSuccess && complete;
+    give_handles(h, complete);
   }
 
   BtData<TV> data(bool mixed) const {
@@ -113,7 +162,8 @@ struct Batch {
 
   bool setup() {
     const unsigned n = in.n;
-    BT_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    if (!take_handles(h)) return false;
+    st = h.st;
     std::vector<int> dims(3 * n);
     std::vector<long> noff(n + 1, 0);
     for (unsigned s = 0; s < n; s++) {
@@ -143,7 +193,6 @@ struct Batch {
       return false;
     const int pmax = 32 * num_sms();  // at most 32 resident CTAs per SM
     if (!buf.alloc(&d_part, ((size_t)pmax + n) * BT_NR)) return false;
-    BT_CK(cudaMallocHost(&h_sch, sizeof(BtSched)));
     BT_CK(cudaMemcpyAsync(d_dims, dims.data(), dims.size() * sizeof(int), cudaMemcpyHostToDevice, st));
     BT_CK(cudaMemcpyAsync(d_noff, noff.data(), noff.size() * sizeof(long), cudaMemcpyHostToDevice, st));
     for (unsigned s = 0; s < n; s++)
@@ -259,8 +308,7 @@ struct Batch {
       p_apply = resident_ctas(k_bt_modal<TV, false>, MD_NT, bt_modal_smem<TV>());
     }
     const int p_point = resident_ctas(k_bt_point<TV, PW_PCG>, PW_NT);
-    cudaEvent_t e0, e1, e2;
-    cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventCreate(&e2);
+    const cudaEvent_t e0 = h.ev[0], e1 = h.ev[1], e2 = h.ev[2];
     bool ok = reset_state();
     cudaEventRecord(e0, st);
     ok = ok && enqueue_schedule<TC>();
@@ -287,9 +335,9 @@ struct Batch {
       for (long c = 0; ok && c < max_chunks; c++) {
         ok = cudaGraphLaunch(gx, st) == cudaSuccess;
         launches += per_graph;
-        ok = ok && cudaMemcpyAsync(h_sch, d_sch, sizeof(BtSched), cudaMemcpyDeviceToHost, st) == cudaSuccess;
+        ok = ok && cudaMemcpyAsync(h.h_sch, d_sch, sizeof(BtSched), cudaMemcpyDeviceToHost, st) == cudaSuccess;
         ok = ok && cudaStreamSynchronize(st) == cudaSuccess;
-        if (ok && h_sch->n_act == 0) break;
+        if (ok && h.h_sch->n_act == 0) break;
       }
     }
     if (!ok && g_err.empty()) g_err = std::string("batch solve: ") + cudaGetErrorString(cudaGetLastError());
@@ -312,7 +360,6 @@ struct Batch {
     }
     if (gx) cudaGraphExecDestroy(gx);
     if (g) cudaGraphDestroy(g);
-    cudaEventDestroy(e0); cudaEventDestroy(e1); cudaEventDestroy(e2);
     return ok;
   }
 
@@ -322,6 +369,7 @@ struct Batch {
     BT_CK(cudaMemcpyAsync(moments, d_mom, (size_t)n * 9 * sizeof(double), cudaMemcpyDeviceToHost, st));
     BT_CK(cudaMemcpyAsync(sc.data(), d_sc, sc.size() * sizeof(DevScalars), cudaMemcpyDeviceToHost, st));
     BT_CK(cudaStreamSynchronize(st));
+    complete = true;
     unsigned maxit = 0, found = 0;
     for (size_t t = 0; t < sc.size(); t++) {
       const DevScalars& h = sc[t];

@@ -24,6 +24,7 @@
 #include "stencil_block.cuh"
 #include "stencil_asm.cuh"
 #include "asm_apply.h"
+#include "devpool.h"
 #include "modal_apply.h"
 #include "modal_point.cuh"
 #include "stencil_2d.cuh"
@@ -183,28 +184,10 @@ static cudapcgFlag_t ctor_simple(cudapcgModel_t** ptr, const void* data) {
 
 template <typename T> static int prec_of() { return sizeof(T) == 8 ? CHFEM_B200_FP64 : CHFEM_B200_MIXED; }
 
-// Device memory of the solver comes from the device's default stream-ordered pool, whose
-// release threshold is raised (to a quarter of the device's memory) so that what one model
-// frees stays mapped for the next: repeated
-// solves (one compute_property call after another) then skip the driver's unmapping and
-// mapping, which cost 0.006 to 0.47 s per 128^3 elastic call on different B200 boxes.
+// Device memory of the solver comes from the device's default stream-ordered pool (devpool.h).
 // cudapcgB200TrimMemory hands the kept blocks back.  Allocations are made on the legacy stream
 // and waited for; a free first waits for the solver's stream, so it follows every launch that
 // may read the block.
-static void pool_keep() {
-  static bool kept[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || kept[dev]) return;
-  cudaMemPool_t pool;
-  size_t free_b = 0, total_b = 0;
-  if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-    // kept at most: a quarter of the device's memory, or CHFEM_B200_POOL_KEEP_BYTES
-    uint64_t threshold = total_b / 4;
-    if (const char* e = getenv("CHFEM_B200_POOL_KEEP_BYTES")) threshold = strtoull(e, nullptr, 10);
-    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
-  }
-  kept[dev] = true;
-}
 template <typename P>
 static cudaError_t dev_malloc(P** p, size_t bytes) {
   pool_keep();

@@ -1,0 +1,27 @@
+// devpool.h -- the device's default stream-ordered memory pool, with its release threshold raised
+// (to a quarter of the device's memory) so that what one call frees stays mapped for the next:
+// repeated solves (one compute_property call after another) then skip the driver's unmapping and
+// mapping, which cost 0.006 to 0.47 s per 128^3 elastic call on different B200 boxes.
+#pragma once
+#include <cuda_runtime.h>
+#include <cstdint>
+#include <cstdlib>
+
+namespace chfem {
+
+inline void pool_keep() {
+  static bool kept[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || kept[dev]) return;
+  cudaMemPool_t pool;
+  size_t free_b = 0, total_b = 0;
+  if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+    // kept at most: a quarter of the device's memory, or CHFEM_B200_POOL_KEEP_BYTES
+    uint64_t threshold = total_b / 4;
+    if (const char* e = getenv("CHFEM_B200_POOL_KEEP_BYTES")) threshold = strtoull(e, nullptr, 10);
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &threshold);
+  }
+  kept[dev] = true;
+}
+
+}  // namespace chfem

@@ -5,6 +5,7 @@
 // the 12-entry scan limit), readMaterialMapRAW/Numpy :1644-1758 (x-fastest file order
 // transposed to the row-fastest internal order, with %refinement replication),
 // hmgSolveHomogenization :848-1198 (solver set-up, direction loop, -xi/-xo files, updateC).
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -937,6 +938,23 @@ int chfemB200LastBatchStats(cudapcgB200BatchStats* out) {
   return 1;
 }
 
+int chfemB200ColorHistogram(const uint8_t* voxels, unsigned long long n, unsigned long long* counts) {
+  if ((!voxels && n) || !counts) { fail("chfemB200ColorHistogram: null argument"); return 0; }
+  for (int c = 0; c < 256; c++) counts[c] = 0;
+#pragma omp parallel if (n > (1u << 16))
+  {
+    // four tables taken in turn, so that a run of one colour does not wait on its own counter
+    std::vector<unsigned long long> h(4 * 256, 0);
+#pragma omp for nowait
+    for (long long i = 0; i < (long long)(n / 4); i++)
+      for (int k = 0; k < 4; k++) h[256 * k + voxels[4 * i + k]]++;
+#pragma omp critical
+    for (int c = 0; c < 256; c++) counts[c] += h[c] + h[256 + c] + h[512 + c] + h[768 + c];
+  }
+  for (unsigned long long i = n / 4 * 4; i < n; i++) counts[voxels[i]]++;
+  return 1;
+}
+
 int chfemB200RunThermalBatch(unsigned int nsamples, const chfemB200ThermalSample* samples, double tol, unsigned int maxit,
                              int precision, double* C_out, unsigned int* iterations, double* solve_seconds) {
   g_err.clear();
@@ -949,8 +967,16 @@ int chfemB200RunThermalBatch(unsigned int nsamples, const chfemB200ThermalSample
   // per sample: voxel material map, node keys and element matrices (the host model layer)
   std::vector<Model> models(nsamples);
   std::vector<int> ok(nsamples, 1);
+  // the largest first: a large sample taken last would leave the other threads idle
+  std::vector<unsigned> order(nsamples);
+  for (unsigned s = 0; s < nsamples; s++) order[s] = s;
+  std::sort(order.begin(), order.end(), [&](unsigned a, unsigned b) {
+    const chfemB200ThermalSample &x = samples[a], &y = samples[b];
+    return (unsigned long long)x.nx * x.ny * x.nz > (unsigned long long)y.nx * y.ny * y.nz;
+  });
 #pragma omp parallel for schedule(dynamic)
-  for (long s = 0; s < (long)nsamples; s++) {
+  for (long o = 0; o < (long)nsamples; o++) {
+    const unsigned s = order[o];
     const chfemB200ThermalSample& t = samples[s];
     Model& m = models[s];
     m.analysis = THERMAL; m.nd = 1; m.C_dim = 9; m.voxel = 1.0; m.refinement = 1; m.tol = tol; m.maxit = maxit;

@@ -111,12 +111,22 @@ bool build_maps(Model& m, std::string& err) {
   if (m.analysis != FLUID) {
     if (m.nmat > 4) { err = "more than 4 materials cannot be encoded in 16-bit node keys"; return false; }
     m.keys.assign(N, 0);
+    // column by column: the voxel in which a node is local node e lies at its row or the one before,
+    // its column or the one before (e = 1, 2), its layer or the one before (e >= 4)
 #pragma omp parallel for schedule(static)
-    for (long i = 0; i < N; i++) {
-      const long r = i % R, c = (i / R) % C, l = i / (R * C);
-      unsigned k = 0;
-      for (int e = 0; e < 8; e++) k |= ((unsigned)m.elem_mat[node_elem(r, c, l, e, R, C, L)] & 3u) << (2 * e);
-      m.keys[i] = (uint16_t)k;
+    for (long col = 0; col < C * L; col++) {
+      const long c = col % C, l = col / C, cm = c ? c - 1 : C - 1, lm = l ? l - 1 : L - 1;
+      const uint16_t* v[4] = {m.elem_mat.data() + (l * C + c) * R, m.elem_mat.data() + (l * C + cm) * R,
+                              m.elem_mat.data() + (lm * C + c) * R, m.elem_mat.data() + (lm * C + cm) * R};
+      for (long r = 0; r < R; r++) {
+        const long rm = r ? r - 1 : R - 1;
+        unsigned k = 0;
+        for (int h = 0; h < 2; h++) {
+          const uint16_t *a = v[2 * h], *b = v[2 * h + 1];
+          k |= ((a[rm] & 3u) | (b[rm] & 3u) << 2 | (b[r] & 3u) << 4 | (a[r] & 3u) << 6) << (8 * h);
+        }
+        m.keys[col * R + r] = (uint16_t)k;
+      }
     }
     m.ndof = N * m.nd;
     return true;

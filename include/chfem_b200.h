@@ -90,6 +90,9 @@ int chfemB200GetSolveStats(chfemB200SolveStats *out);
 int chfemB200Run(const uint8_t *voxels, const char *nf, int direction, int solver, int precondition,
                  int precision, int multirhs, double *C_out);
 
+/* Voxels of each colour of an image of n bytes: counts[256].  Returns 1, or 0 on a null argument. */
+int chfemB200ColorHistogram(const uint8_t *voxels, unsigned long long n, unsigned long long *counts);
+
 /* Batched thermal homogenization of many independent images (no counterpart in the reference,
    which homogenizes one image per run): sample s is an nx*ny*nz uint8 image in C order of a
    (z,y,x) array (the .raw layout), whose colours colors[0..nmat-1] have conductivities

@@ -40,3 +40,28 @@ def test_compute_property_argument_errors():
         compute_property("conductivity", a + 3, mat_props={3: 1.0})
     with pytest.raises(ValueError, match="Material properties"):
         compute_property("conductivity", a)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 5, 7), (2, 40, 33), (17, 64, 128)])
+def test_colour_histogram_equals_bincount(shape):
+    """The native count (threads over chunks of the image) is numpy's for every size and colour."""
+    from chfem_b200.io import _color_histogram
+    img = np.random.default_rng(5).integers(0, 256, size=shape).astype(np.uint8)
+    for a in (img, np.full(shape, 255, np.uint8)):
+        hist = _color_histogram(a)
+        assert hist.dtype == np.int64 and np.array_equal(hist, np.bincount(a.reshape(-1), minlength=256))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 2, 3), (4, 1, 5), (3, 5, 1), (6, 7, 9)])
+def test_node_keys_name_the_eight_voxels(tmp_path, shape):
+    """2 bits per local node e: the material of the voxel in which the node is corner e, on the
+    periodic grid (x: +columns, y: -rows, z: -layers; nodes stored rows fastest)."""
+    from tests.test_gpu_parity import host_arrays
+    img = H.small_image(shape, 4, seed=3)
+    nf, raw = H.write_small_case(str(tmp_path), "keys", img, 0)
+    keys = host_arrays(nf, raw)["keys"]
+    mat = np.searchsorted(np.unique(img), img).transpose(0, 2, 1)  # (layers, columns, rows)
+    ref = np.zeros(mat.shape, np.int64)
+    for e, (dl, dc, dr) in enumerate([(0, 0, 1), (0, 1, 1), (0, 1, 0), (0, 0, 0), (1, 0, 1), (1, 1, 1), (1, 1, 0), (1, 0, 0)]):
+        ref |= np.roll(mat, (dl, dc, dr), axis=(0, 1, 2)) << (2 * e)
+    assert np.array_equal(keys, ref.reshape(-1))
