@@ -1146,6 +1146,15 @@ static bool upload_vec(const double* host, void* dst_T) {
   return true;
 }
 
+// A vector of nvars doubles into a buffer that was zeroed on the solver's stream, after that
+// zeroing (the legacy stream, on which the copy follows the caller's own work, does not wait for
+// the solver's).
+static bool copy_in(double* dst, const double* src, cudaMemcpyKind kind) {
+  CKV(cudaStreamSynchronize(S->stream));
+  CKV(cudaMemcpy(dst, src, (size_t)S->nvars * 8, kind));
+  return true;
+}
+
 static bool ensure_vectors_current() {
   if (lean_solver()) return ensure_lean_vectors();
   return (S->precision == CHFEM_B200_FP64) ? ensure_vectors<double>() : ensure_vectors<float>();
@@ -1155,7 +1164,7 @@ cudapcgFlag_t cudapcgSetRHS(cudapcgVar_t* RHS) {
   if (!S || !S->model || !RHS) return CUDAPCG_FALSE;
   if (!ensure_vectors_current()) return CUDAPCG_FALSE;
   if (lean_solver()) {  // the 2-vector solvers consume r in place; no other copy is kept
-    CK(cudaMemcpy(S->r, RHS, S->nvars * 8, cudaMemcpyHostToDevice));
+    if (!copy_in((double*)S->r, RHS, cudaMemcpyHostToDevice)) return CUDAPCG_FALSE;
     S->rhs_set = true;
     return CUDAPCG_TRUE;
   }
@@ -1226,7 +1235,7 @@ extern "C" {
 cudapcgFlag_t cudapcgB200SetX0Device(const double* x0) {
   if (!S || !S->model || !x0) return CUDAPCG_FALSE;
   if (!ensure_vectors_current()) return CUDAPCG_FALSE;
-  CK(cudaMemcpy(lean_solver() ? (double*)S->d0 : S->x, x0, S->nvars * 8, cudaMemcpyDeviceToDevice));
+  if (!copy_in(lean_solver() ? (double*)S->d0 : S->x, x0, cudaMemcpyDeviceToDevice)) return CUDAPCG_FALSE;
   S->x0_set = true;
   return CUDAPCG_TRUE;
 }
@@ -1241,13 +1250,13 @@ cudapcgFlag_t cudapcgSetX0(cudapcgVar_t* x0, cudapcgFlag_t mustInterpolate) {
   if (!ensure_vectors_current()) return CUDAPCG_FALSE;
   if (lean_solver()) {  // the 2-vector solvers hold x0 in d (cudapcg.cu:302)
     if (mustInterpolate) { set_err("cudapcgSetX0", "coarse-grid guesses are not provided for Stokes"); return CUDAPCG_FALSE; }
-    CK(cudaMemcpy(S->d0, x0, S->nvars * 8, cudaMemcpyHostToDevice));
+    if (!copy_in((double*)S->d0, x0, cudaMemcpyHostToDevice)) return CUDAPCG_FALSE;
     S->x0_set = true;
     return CUDAPCG_TRUE;
   }
   bool ok;
   if (mustInterpolate) ok = (S->vec_prec == CHFEM_B200_FP64) ? interp_x0<double>(x0) : interp_x0<float>(x0);
-  else { ok = cudaMemcpy(S->x, x0, S->nvars * 8, cudaMemcpyHostToDevice) == cudaSuccess; }
+  else ok = copy_in(S->x, x0, cudaMemcpyHostToDevice);
   if (!ok) return CUDAPCG_FALSE;
   S->x0_set = true;
   return CUDAPCG_TRUE;
