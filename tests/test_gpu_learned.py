@@ -103,3 +103,29 @@ def test_compute_property_with_learned_guess(multirhs):
     assert H.rel_to_max(C1, C0) < 1e-6
     with pytest.raises(ValueError):
         compute_property("elasticity", img[:, :, :30], initial_guess="learned", **kw)
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 8, 8), (1, 8, 8, 40), (3, 16, 8, 24), (1, 40, 24, 8), (2, 24, 40, 32)])
+def test_network_at_tile_edges(shape):
+    """Forward and gradients at sizes that leave parts of the 8-position groups' tiles and of the
+    weight gradient's slabs empty; bars as above, per layer."""
+    import torch
+    import learned_oracle as LO
+    from chfem_b200 import learned as L
+    N, D, Hh, W = shape
+    rng = np.random.default_rng(D + W)
+    net = L.Net(seed=1)
+    net.p.copy_(torch.tensor(rng.standard_normal(net.p.numel()) * 0.15, dtype=torch.float32))
+    p = net.p.cpu().numpy().astype(np.float64)
+    feat, gout = rng.standard_normal((N, 2, D, Hh, W)), rng.standard_normal((N, L.OUT_CH, D, Hh, W))
+    out = net.forward(torch.tensor(feat, dtype=torch.float32, device="cuda")).cpu().numpy()
+    net.backward(torch.tensor(gout, dtype=torch.float32, device="cuda"))
+    g = net.g.cpu().numpy().astype(np.float64)
+    gref = np.zeros_like(p)
+    for n in range(N):
+        o = LO.UNet(p)
+        assert H.rel_to_max(out[n], o.forward(feat[n])) < 1e-4
+        gref += o.backward(gout[n])
+    for name, (w0, b0, co, ci, k) in LO.offsets()[0].items():
+        assert H.rel_to_max(g[w0:b0], gref[w0:b0]) < 1e-3, name
+        assert H.rel_to_max(g[b0:b0 + co], gref[b0:b0 + co]) < 1e-3, name
