@@ -408,12 +408,13 @@ def batch_main(args, w, world, rank, dist, allmax, barrier):
     per_unit = 12 * es + 2
     peak, peak_kind = load_peaks()
     tile = {4: 0, 8: 1, 16: 2}.get(st0.tile_cols, 1)
+    modal = st0.tile_ms[0] == 0  # isotropic batches run one tile shape in voxel modes
     kt = st0.tile_ms[tile] * 1e-3 if st0.tile_ms[tile] > 0 else None
     achieved = per_unit * nodes / kt / 1e9 if kt else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak if achieved else None, "traffic": profiled_traffic(args.workload),
-                "kernel": f"k_bt_apply<{st0.tile_cols},{'float' if es == 4 else 'double'},false> (batch operator + directions + dots, "
-                          f"{w['batch']} samples x 3 load cases; tile 32x{st0.tile_cols} chosen by the autotuner)",
+                "kernel": f"{'k_bt_modal<' if modal else f'k_bt_apply<{st0.tile_cols},'}{'float' if es == 4 else 'double'},false> (batch operator + "
+                          f"directions + dots, {w['batch']} samples x 3 load cases; tile 32x{st0.tile_cols})",
                 "kernel_ms": kt * 1e3 if kt else None, "bytes_per_unit": per_unit, "units_per_launch": nodes,
                 "tile_ms_4_8_16": list(st0.tile_ms), "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"}
     node_its = float(sum(imgs[i].size * int(its[i].sum()) for i in range(len(imgs))))
@@ -754,28 +755,28 @@ def dominant_kernel_roofline(model, w, block, workload):
     peak, peak_kind = load_peaks()
     es = 4 if w["precision"] == "mixed" else 8
     if w["analysis"] == 2:
-        kern_which, kname = 3, "k_fl_apply<MR> (Stokes operator + PMINRES step, one right-hand side)"
-        # per DOF: r, q, d in, q', r' out (5 es) and the FP64 x read and written (16 B); per row
-        # set (pore node: 4 DOFs, interface node: 1) its DOF->node and node->DOF entries (8 B) and
+        kern_which, kname = 3, "k_fl_mr_upd + k_fl_mr_apply (Stokes PMINRES step and operator, one right-hand side)"
+        # per DOF: r, x read and written, q, d read; z written and read; s written, r read again (10 x
+        # 8 B); per row set (pore node: 4 DOFs, interface node: 1) its DOF->node entry twice (8 B) and
         # an interface node's fluid key (1 B); units = row sets, bytes_per_unit their mean
         nV, nB = model.info[5], model.info[6]
         units = nV + nB
-        per_unit = (nV * (4 * (5 * es + 16) + 8) + nB * ((5 * es + 16) + 9)) / max(1, units)
+        per_unit = (nV * (4 * 80 + 8) + nB * (80 + 9)) / max(1, units)
     else:
         nd = 3 if w["analysis"] == 1 else 1
         tn = 'float' if es == 4 else 'double'
         if block:
             nr = 6 if nd == 3 else 3
-            asm = model.nmat <= 2 and os.environ.get("CHFEM_B200_BLOCK_OP") != "element"
+            modal = os.environ.get("CHFEM_B200_BLOCK_OP") != "element"
             kern_which = 5
-            kname = (f"k_asm_apply<{nd},{tn},{nr}> (block operator, stencil assembled per material configuration, "
-                     f"+ directions + dots, {nr} load cases)" if asm else
+            vt = "float2" if es == 4 and nr % 2 == 0 else tn
+            kname = (f"k_modal_apply<{nd},{vt},TE_PCG> block (operator in voxel modes + directions + dots, {nr} load cases)" if modal else
                      f"k_blk_apply<{nd},{tn},{nr}> (block operator + directions + dots, {nr} load cases)")
             per_unit = nr * 4 * nd * es + 2  # per load case s, d_old in; d_new, q out; one 16-bit key
-        elif nd == 1 and model.nmat <= 4 and os.environ.get("CHFEM_B200_THERMAL_OP") != "generic":
+        elif os.environ.get("CHFEM_B200_THERMAL_OP" if nd == 1 else "CHFEM_B200_BLOCK_OP") not in ("generic", "element"):
             kern_which = 1
-            kname = f"k_th_apply<{tn},TE_PCG> (thermal operator for cubic-symmetric conduction matrices + direction + dot)"
-            per_unit = 4 * es + 2
+            kname = f"k_modal_apply<{nd},{tn},TE_PCG> (operator in voxel modes + direction + dot)"
+            per_unit = 4 * nd * es + 2
         else:
             kern_which, kname = 1, f"k_te_apply<{nd},{tn},TE_PCG> (operator + direction + dot)"
             per_unit = 4 * nd * es + 2  # s, d_old in; d_new, q out (nd comps); 16-bit key
