@@ -408,13 +408,12 @@ def batch_main(args, w, world, rank, dist, allmax, barrier):
     per_unit = 12 * es + 2
     peak, peak_kind = load_peaks()
     tile = {4: 0, 8: 1, 16: 2}.get(st0.tile_cols, 1)
-    modal = st0.tile_ms[0] == 0  # isotropic batches run one tile shape in voxel modes
     kt = st0.tile_ms[tile] * 1e-3 if st0.tile_ms[tile] > 0 else None
     achieved = per_unit * nodes / kt / 1e9 if kt else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak if achieved else None, "traffic": profiled_traffic(args.workload),
-                "kernel": f"{'k_bt_modal<' if modal else f'k_bt_apply<{st0.tile_cols},'}{'float' if es == 4 else 'double'},false> (batch operator + "
-                          f"directions + dots, {w['batch']} samples x 3 load cases; tile 32x{st0.tile_cols})",
+                "kernel": f"k_bt_apply<{st0.tile_cols},{'float' if es == 4 else 'double'},false> (batch operator + directions + dots, "
+                          f"{w['batch']} samples x 3 load cases; tile 32x{st0.tile_cols} chosen by the autotuner)",
                 "kernel_ms": kt * 1e3 if kt else None, "bytes_per_unit": per_unit, "units_per_launch": nodes,
                 "tile_ms_4_8_16": list(st0.tile_ms), "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"}
     node_its = float(sum(imgs[i].size * int(its[i].sum()) for i in range(len(imgs))))

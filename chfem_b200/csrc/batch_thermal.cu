@@ -99,9 +99,9 @@ int num_sms() {
   return n;
 }
 template <typename K>
-int resident_ctas(K kernel, int threads, size_t smem = 0) {
+int resident_ctas(K kernel, int threads) {
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
   return per_sm * num_sms();
 }
 
@@ -129,8 +129,7 @@ struct Batch {
   long* d_noff = nullptr;
   uint16_t* d_keys = nullptr;
   TV* d_K = nullptr;
-  double* d_lam = nullptr;  // per sample and material: the constant of the voxel modes (all isotropic)
-  bool modal = false;
+  bool iso = false;  // every conductivity matrix is isotropic
   double *d_K64 = nullptr, *d_CB = nullptr, *d_x = nullptr, *d_b = nullptr, *d_part = nullptr, *d_mom = nullptr;
   TV *d_r = nullptr, *d_s = nullptr, *d_d0 = nullptr, *d_d1 = nullptr, *d_q = nullptr;
   DevScalars* d_sc = nullptr;
@@ -149,7 +148,7 @@ struct Batch {
 
   BtData<TV> data(bool mixed) const {
     BtData<TV> a;
-    a.n = (int)in.n; a.dims = d_dims; a.noff = d_noff; a.keys = d_keys; a.K = d_K; a.K64 = d_K64; a.lam = modal ? d_lam : nullptr;
+    a.n = (int)in.n; a.dims = d_dims; a.noff = d_noff; a.keys = d_keys; a.K = d_K; a.K64 = d_K64; a.iso = iso;
     a.sc = d_sc; a.ctl = d_ctl; a.sch = d_sch; a.act = d_act; a.wpre = d_wpre; a.npre = d_npre;
     a.part = d_part; a.ticket = d_ticket; a.pending = &d_sch->pending;
     a.cfg.tol = in.tol; a.cfg.maxit = (int)std::min<unsigned>(in.maxit, 0x7fffffffu); a.cfg.norm = NORM_L2;
@@ -177,16 +176,13 @@ struct Batch {
       for (unsigned t = 0; t < 64 * in.nmat[s]; t++) { K64[(size_t)s * 256 + t] = in.K[s][t]; Kv[(size_t)s * 256 + t] = TV(in.K[s][t]); }
       for (unsigned t = 0; t < 24 * in.nmat[s]; t++) CB[(size_t)s * 96 + t] = in.CB[s][t];
     }
-    std::vector<double> lam((size_t)n * 4, 0.0), tab((size_t)md_table_words());
-    modal = true;
-    for (unsigned s = 0; s < n && modal; s++) {
-      modal = md_build_table(1, (int)in.nmat[s], in.K[s], tab.data()) && md_layer_fits(1, in.dims[3 * s], in.dims[3 * s + 1]);
-      for (unsigned m = 0; m < in.nmat[s]; m++) lam[4 * s + m] = tab[MD_MAT + 2 * m];
-    }
+    std::vector<double> tab((size_t)md_table_words());
+    iso = true;
+    for (unsigned s = 0; s < n && iso; s++) iso = md_build_table(1, (int)in.nmat[s], in.K[s], tab.data());
     const size_t nv = (size_t)BT_NR * Ntot;
-    if (!buf.alloc(&d_lam, 4 * n) || !buf.alloc(&d_dims, 3 * n) || !buf.alloc(&d_noff, n + 1) || !buf.alloc(&d_keys, Ntot) || !buf.alloc(&d_K, (size_t)n * 256) ||
+    if (!buf.alloc(&d_dims, 3 * n) || !buf.alloc(&d_noff, n + 1) || !buf.alloc(&d_keys, Ntot) || !buf.alloc(&d_K, (size_t)n * 256) ||
         !buf.alloc(&d_K64, (size_t)n * 256) || !buf.alloc(&d_CB, (size_t)n * 96) || !buf.alloc(&d_x, nv) || !buf.alloc(&d_b, nv) ||
-        !buf.alloc(&d_r, nv) || (!modal && !buf.alloc(&d_s, nv)) || !buf.alloc(&d_d0, nv) || !buf.alloc(&d_d1, nv) || !buf.alloc(&d_q, nv) ||
+        !buf.alloc(&d_r, nv) || !buf.alloc(&d_s, nv) || !buf.alloc(&d_d0, nv) || !buf.alloc(&d_d1, nv) || !buf.alloc(&d_q, nv) ||
         !buf.alloc(&d_sc, (size_t)BT_NR * n) || !buf.alloc(&d_ctl, (size_t)BT_NR * n) || !buf.alloc(&d_sch, 1) ||
         !buf.alloc(&d_act, n) || !buf.alloc(&d_wpre, n + 1) || !buf.alloc(&d_npre, n + 1) || !buf.alloc(&d_ticket, 1) ||
         !buf.alloc(&d_mom, (size_t)n * 9))
@@ -197,7 +193,6 @@ struct Batch {
     BT_CK(cudaMemcpyAsync(d_noff, noff.data(), noff.size() * sizeof(long), cudaMemcpyHostToDevice, st));
     for (unsigned s = 0; s < n; s++)
       BT_CK(cudaMemcpyAsync(d_keys + noff[s], in.keys[s], (noff[s + 1] - noff[s]) * sizeof(uint16_t), cudaMemcpyHostToDevice, st));
-    BT_CK(cudaMemcpyAsync(d_lam, lam.data(), lam.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     BT_CK(cudaMemcpyAsync(d_K64, K64.data(), K64.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     BT_CK(cudaMemcpyAsync(d_K, Kv.data(), Kv.size() * sizeof(TV), cudaMemcpyHostToDevice, st));
     BT_CK(cudaMemcpyAsync(d_CB, CB.data(), CB.size() * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -213,7 +208,7 @@ struct Batch {
   bool reset_state() {
     const size_t nv = (size_t)BT_NR * Ntot;
     BT_CK(cudaMemsetAsync(d_x, 0, nv * sizeof(double), st));
-    if (d_s) BT_CK(cudaMemsetAsync(d_s, 0, nv * sizeof(TV), st));
+    BT_CK(cudaMemsetAsync(d_s, 0, nv * sizeof(TV), st));
     BT_CK(cudaMemsetAsync(d_d0, 0, nv * sizeof(TV), st));
     BT_CK(cudaMemsetAsync(d_d1, 0, nv * sizeof(TV), st));
     BT_CK(cudaMemsetAsync(d_q, 0, nv * sizeof(TV), st));
@@ -236,13 +231,11 @@ struct Batch {
     TV* dnew = parity ? d_d0 : d_d1;
     const BtData<TV> a = data(mixed);
     const dim3 blk(TE_TR, TC);
-    if (modal) k_bt_modal<TV, false><<<p_apply, MD_NT, bt_modal_smem<TV>(), st>>>(a, d_r, dold, dnew, d_q, d_x, d_b, d_r);
-    else k_bt_apply<TC, TV, false><<<p_apply, blk, 0, st>>>(a, d_s, dold, dnew, d_q, d_x, d_b, d_r);
+    k_bt_apply<TC, TV, false><<<p_apply, blk, 0, st>>>(a, d_s, dold, dnew, d_q, d_x, d_b, d_r);
     k_bt_point<TV, PW_PCG><<<p_point, PW_NT, 0, st>>>(a, d_x, dnew, d_r, d_q, d_s);
     launches += 2;
     if (mixed) {
-      if (modal) k_bt_modal<TV, true><<<p_apply, MD_NT, bt_modal_smem<double>(), st>>>(a, d_s, dold, dnew, d_q, d_x, d_b, d_r);
-      else k_bt_apply<TC, TV, true><<<p_apply, blk, 0, st>>>(a, d_s, dold, dnew, d_q, d_x, d_b, d_r);
+      k_bt_apply<TC, TV, true><<<p_apply, blk, 0, st>>>(a, d_s, dold, dnew, d_q, d_x, d_b, d_r);
       k_bt_point<TV, PW_REPL><<<p_point, PW_NT, 0, st>>>(a, d_x, dnew, d_r, d_q, d_s);
       launches += 2;
     }
@@ -274,39 +267,9 @@ struct Batch {
     return ok ? best : 1e30;
   }
 
-  // the same for the pass in voxel modes
-  double time_modal() {
-    if (cudaFuncSetAttribute(k_bt_modal<TV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_modal_smem<TV>()) != cudaSuccess) return 0.0;
-    const int p = resident_ctas(k_bt_modal<TV, false>, MD_NT, bt_modal_smem<TV>());
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    float best = 1e30f;
-    bool ok = reset_state() && enqueue_schedule<MD_TC>();
-    for (int rep = 0; ok && rep < 3; rep++) {
-      cudaEventRecord(e0, st);
-      k_bt_modal<TV, false><<<p, MD_NT, bt_modal_smem<TV>(), st>>>(data(false), d_r, d_d0, d_d1, d_q, d_x, d_b, d_r);
-      cudaEventRecord(e1, st);
-      ok = cudaEventSynchronize(e1) == cudaSuccess;
-      float ms = 0;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (rep > 0) best = std::min(best, ms);
-    }
-    launches += 3;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    return ok ? best : 0.0;
-  }
-
   template <int TC>
   bool solve(bool mixed, cudapcgB200BatchStats* stats) {
-    int p_apply = modal ? 0 : resident_ctas(k_bt_apply<TC, TV, false>, TE_TR * TC);
-    if (modal) {
-      // above 48 KB of shared memory the kernels ask for it
-      BT_CK(cudaFuncSetAttribute(k_bt_modal<TV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_modal_smem<TV>()));
-      BT_CK(cudaFuncSetAttribute(k_bt_modal<TV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_modal_smem<double>()));
-      p_apply = resident_ctas(k_bt_modal<TV, false>, MD_NT, bt_modal_smem<TV>());
-    }
+    const int p_apply = resident_ctas(k_bt_apply<TC, TV, false>, TE_TR * TC);
     const int p_point = resident_ctas(k_bt_point<TV, PW_PCG>, PW_NT);
     const cudaEvent_t e0 = h.ev[0], e1 = h.ev[1], e2 = h.ev[2];
     bool ok = reset_state();
@@ -398,14 +361,6 @@ int run_batch(const Inputs& in, bool mixed, double* moments, unsigned* iteration
   }
   int tc;
   auto it = g_tile_cache.find(sig);
-  if (b.modal) {  // one tile shape; its pass timed once per signature, for the statistics
-    if (it == g_tile_cache.end()) {
-      const double t = b.time_modal();
-      if (stats) stats->tile_ms[1] = t;
-      g_tile_cache[sig] = MD_TC;
-    }
-    return b.template solve<MD_TC>(mixed, stats) ? (b.results(moments, iterations, residuals, stats) ? 1 : 2) : 0;
-  }
   if (it != g_tile_cache.end()) tc = it->second;
   else {
     const double t4 = b.template time_apply<4>(), t8 = b.template time_apply<8>(), t16 = b.template time_apply<16>();

@@ -28,7 +28,6 @@
 #include "pointwise.cuh"
 #include "stencil_te.cuh"
 #include "stencil_block.cuh"
-#include "stencil_modal.cuh"
 #include "loadcase.cuh"
 
 namespace chfem {
@@ -64,7 +63,7 @@ struct BtData {
   const uint16_t* keys;      // [noff[n]]
   const TV* K;               // [n][4][64] dense conductivity matrices (slots past nmat zero)
   const double* K64;         // same in FP64 (replacement operator, right-hand sides)
-  const double* lam;         // [n][4] constants of the voxel modes (k / 16 per material), or null
+  int iso;                   // every conductivity matrix is isotropic (one diagonal value per material)
   DevScalars* sc;            // [n][3]
   BtCtl* ctl;                // [n][3]
   const BtSched* sch;
@@ -335,171 +334,13 @@ __global__ void __launch_bounds__(TE_TR * TC) k_bt_apply(BtData<TV> a, const TV*
   bt_finish_alpha<TV, NT>(a, sch, P, W);
 }
 
-// The same pass in voxel modes (stencil_modal.cuh), for batches whose conductivity matrices are
-// all isotropic: 32 x 8 columns, a thread per node of the haloed plane, the sample's three load
-// cases together (they share the node's key and all index arithmetic).  sv: r, of which M^-1 r is formed
-// here and never stored.  A load case that does not take part is neither read nor written.
-constexpr int BM_CW = MD_PR * (MD_TC + 1);  // one corner's forces of a plane
-template <typename TS>
-inline size_t bt_modal_smem() { return (size_t)BT_NR * (4 * MD_PP + 8 * BM_CW) * sizeof(TS); }
-
-template <typename TV, bool RES>
-__global__ void __launch_bounds__(MD_NT, (RES || sizeof(TV) == 8) ? 1 : 2) k_bt_modal(BtData<TV> a, const TV* sv, const TV* dold, TV* dnew, TV* q,
-                                                                                       const double* x, const double* b64, TV* r) {
-  using TS = std::conditional_t<RES, double, TV>;  // staging / compute type
-  constexpr int NT = MD_NT, PP = MD_PP, PR = MD_PR, CW = BM_CW;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  TS* sP = reinterpret_cast<TS*>(smem_raw);  // [4][BT_NR][PP] formed input
-  TS* sC = sP + 4 * BT_NR * PP;              // [2][4][BT_NR][CW] corner forces
-  __shared__ double sred[NT / 32];
-  __shared__ TS sbeta[BT_NR], slam[4];
-  __shared__ BtDiag<TS> sdiag;
-  __shared__ int son[BT_NR];  // load case served by this pass
-  const BtSched sch = *a.sch;
-  if (sch.n_act == 0 || (RES && !sch.pending)) return;
-  const int P = gridDim.x, bid = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-  const long W = sch.W, w0 = (long)bid * W / P, w1 = ((long)bid + 1) * W / P;
-  const int vr = tid % PR, vc = tid / PR;
-  const bool point = tid < PP, voxel = vr < PR - 1 && vc < MD_TC + 1;
-  double acc[BT_NR] = {0.0, 0.0, 0.0};
-  int cur = -1, s = 0, R = 1, C = 1, L = 1, tiles_r = 1;
-  long nbase = 0, vbase = 0, Ns = 0;
-  bool on[BT_NR] = {false, false, false};
-  auto flush = [&](int i) {
-    if constexpr (!RES) {
-#pragma unroll
-      for (int k = 0; k < BT_NR; k++) {
-        const double t = block_sum<NT>(acc[k], sred);
-        if (tid == 0) a.part[((long)bid + i) * BT_NR + k] = t;
-        acc[k] = 0.0;
-      }
-    }
-  };
-  int i = (w0 < w1) ? bt_find(a.wpre, sch.n_act, w0) : 0;
-  for (long w = w0; w < w1;) {
-    while (w >= a.wpre[i + 1]) i++;
-    if (i != cur) {
-      if (cur >= 0) flush(cur);
-      cur = i;
-      s = a.act[i];
-      R = a.dims[3 * s]; C = a.dims[3 * s + 1]; L = a.dims[3 * s + 2];
-      tiles_r = (R + TE_TR - 1) / TE_TR;
-      nbase = a.noff[s]; Ns = (long)R * C * L; vbase = BT_NR * nbase;
-      __syncthreads();
-      if (tid < 4) slam[tid] = TS(a.lam[4 * s + tid]);
-      if (!RES) bt_diag_fill<TS>(sdiag, a.K64 + (size_t)s * 256, tid, a.cfg.precond != 0);
-      if (tid < BT_NR) {
-        const DevScalars& scs = a.sc[BT_NR * s + tid];
-        if (RES) son[tid] = a.ctl[BT_NR * s + tid].pending != BT_NONE;
-        else son[tid] = !scs.done;
-        sbeta[tid] = RES ? TS(0) : TS(scs.beta);
-      }
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < BT_NR; k++) on[k] = son[k];
-    }
-    const long u = w - a.wpre[i];
-    const int tile = (int)(u / L), l0 = (int)(u - (long)tile * L);
-    const int l1 = (int)min((long)L, (long)l0 + (min(w1, a.wpre[i + 1]) - w));
-    w += l1 - l0;
-    if (!(on[0] || on[1] || on[2])) continue;
-    const int r0 = (tile % tiles_r) * TE_TR, c0 = (tile / tiles_r) * MD_TC;
-    const long RC = (long)R * C;
-    const int node = point ? wrap(r0 + vr - 1, R) + wrap(c0 + vc - 1, C) * R : 0;
-    const bool act = wp < MD_TC && c0 + wp < C && r0 + lane < R;
-    const int onode = r0 + lane + (c0 + wp) * R;
-    auto first = [&](int l) { return (long)(l < 0 ? l + L : (l >= L ? l - L : l)) * RC; };
-    TS g0[BT_NR], g1[BT_NR];
-    unsigned gk = 0, vmat = 0;
-    auto load = [&](int l) {
-      if (!point) return;
-      const long j0 = first(l) + node;
-      gk = a.keys[nbase + j0];
-#pragma unroll
-      for (int k = 0; k < BT_NR; k++) {
-        if (!on[k]) continue;
-        const long j = vbase + k * Ns + j0;
-        if (RES) g0[k] = TS(x[j]);
-        else { g0[k] = TS(sv[j]); g1[k] = TS(dold[j]); }
-      }
-    };
-    TS mo[BT_NR][4], fc[BT_NR][1][4];
-#pragma unroll
-    for (int k = 0; k < BT_NR; k++) g0[k] = g1[k] = TS(0);
-    __syncthreads();  // the previous run's reads of the planes are done
-    load(l0 - 1);
-    for (int l = l0 - 1; l <= l1 + 1; l++) {
-      TS v[BT_NR];
-      unsigned vnext = 0;
-      if (l <= l1) {
-        vnext = md_material(gk);
-        const TS inv = RES ? TS(1) : bt_inv<TS>(sdiag, gk);
-#pragma unroll
-        for (int k = 0; k < BT_NR; k++) {
-          v[k] = RES ? g0[k] : TS(fma(sbeta[k], g1[k], inv * g0[k]));
-          if (point) sP[((l & 3) * BT_NR + k) * PP + tid] = v[k];
-        }
-        if (l < l1) load(l + 1);
-      }
-      __syncthreads();
-      if (l <= l1 && voxel) {
-        const TS lam = slam[vmat];
-#pragma unroll
-        for (int k = 0; k < BT_NR; k++) {
-          if (!on[k]) continue;
-          const TS* pl = sP + ((l & 3) * BT_NR + k) * PP + tid;
-          TS nm[1][4];
-          md_plane<TS>(v[k], pl[1], pl[PR], pl[PR + 1], nm[0]);
-          if (l >= l0) {
-            TS ms[1][4], mdif[1][4], fa[1][4];
-            md_layers<TS>(mo[k], nm[0], ms[0], mdif[0]);
-            md_voxel<1, TS, TS>(ms, mdif, lam, lam, fc[k], fa);
-            if (l > l0) {
-              TS* f = sC + ((l & 1) * 4 * BT_NR + k) * CW + tid;
-              TS f00, f10, f01, f11;
-              md_plane_t<TS>(fa[0], f00, f10, f01, f11);
-              f[0] = f00;
-              f[BT_NR * CW] = f10;
-              f[2 * BT_NR * CW] = f01;
-              f[3 * BT_NR * CW] = f11;
-            }
-          } else {
-#pragma unroll
-            for (int m = 0; m < 4; m++) fc[k][0][m] = TS(0);
-          }
-#pragma unroll
-          for (int m = 0; m < 4; m++) mo[k][m] = nm[0][m];
-        }
-      }
-      vmat = vnext;
-      if (l - 2 >= l0 && act) {
-        const long j0 = first(l - 2) + onode;
-#pragma unroll
-        for (int k = 0; k < BT_NR; k++) {
-          if (!on[k]) continue;
-          const TS* f = sC + (((l - 1) & 1) * 4 * BT_NR + k) * CW + wp * PR + lane;
-          const TS out = (f[PR + 1] + f[BT_NR * CW + PR]) + (f[2 * BT_NR * CW + 1] + f[3 * BT_NR * CW]);
-          const long j = vbase + k * Ns + j0;
-          if (RES) {
-            r[j] = TV(b64[j] - (double)out);
-          } else {
-            const TS vv = sP[(((l - 2) & 3) * BT_NR + k) * PP + (wp + 1) * PR + lane + 1];
-            q[j] = TV(out);
-            dnew[j] = TV(vv);
-            acc[k] += (double)vv * (double)out;
-          }
-        }
-      }
-    }
-  }
-  if (RES) return;
-  if (cur >= 0) flush(cur);
-  bt_finish_alpha<TV, NT>(a, sch, P, W);
-}
-
 // Pointwise pass over the node line of the active samples.
-// A thread takes 4 nodes of every load case (16-byte accesses where the sample's vectors allow
-// them); sv null: s = M^-1 r is not stored (the modal operator forms it).
+// A thread takes 4 nodes of every load case, with 16-byte accesses where the sample's vectors allow
+// them: bound by HBM, where one word per access and 8 divisions a node were not (24 images of 32^3
+// to 96^3, FP32 fields: 203 -> 147 ms a solve with the finishers by warps).
+// Its operator stays the general one: in voxel modes (stencil_modal.cuh, three load cases a thread, M^-1 r
+// formed from r) it took 0.48 ms a pass against 0.34, as 80 registers a thread do not hold three
+// cases' layers.
 //   PW_INIT: s = M^-1 r, delta0 (zero guess); PW_PCG: x += a d, r -= a q, s = M^-1 r, delta,
 //   stopping test (and, mixed, the replacement / check decisions); PW_REPL: for pending load
 //   cases, s = M^-1 r from the true residual, then the replacement or check finisher.
@@ -514,7 +355,7 @@ __global__ void __launch_bounds__(PW_NT) k_bt_point(BtData<TV> a, double* x, con
   if (sch.n_act == 0 || (MODE == PW_REPL && !sch.pending)) return;
   const int P = gridDim.x, bid = blockIdx.x, tid = threadIdx.x;
   const long Nn = sch.Nn, n0 = (long)bid * Nn / P, n1 = ((long)bid + 1) * Nn / P;
-  const bool iso = a.lam != nullptr;
+  const bool iso = a.iso;
   double acc[BT_NR] = {0.0, 0.0, 0.0};
   int cur = -1;
   auto flush = [&](int i) {
@@ -607,13 +448,13 @@ __global__ void __launch_bounds__(PW_NT) k_bt_point(BtData<TV> a, double* x, con
           }
           if (vec) {
             if (MODE == PW_PCG) { blk_st4(x + j, xv); blk_st4(r + j, rv); }
-            if (sv) blk_st4(sv + j, sn);
+            blk_st4(sv + j, sn);
           } else {
 #pragma unroll
             for (int u = 0; u < 4; u++) {
               if (u >= m) break;
               if (MODE == PW_PCG) { x[j + u] = xv[u]; r[j + u] = rv[u]; }
-              if (sv) sv[j + u] = sn[u];
+              sv[j + u] = sn[u];
             }
           }
         }

@@ -191,8 +191,7 @@ cudapcgFlag_t cudapcgB200SolveLoadCases(unsigned int nrhs, const int *axis, cons
    Out: moments[9s + 3k + row] = sum over voxels of (CB x_k)_row for load case k (add the face
    term and divide by the voxel count for the tensor); iterations/residuals [3s + k] may be NULL.
    precision CHFEM_B200_FP64 or CHFEM_B200_MIXED (FP32 fields; FP64 x, dots, replacement).
-   Batches of isotropic materials run the operator in voxel modes (32 x 8 nodes, its pass timed once
-   per batch signature); otherwise the tile shape (32 x 4, 8 or 16 nodes) is timed once per batch signature and
+   The operator's tile shape (32 x 4, 8 or 16 nodes) is timed once per batch signature and
    remembered.  Returns 1 when every load case converged, 2 when some stopped at maxit, 0 on
    error (cudapcgB200BatchLastError).  Independent of the cudapcgInit model. */
 typedef struct {

@@ -90,9 +90,9 @@ def test_batch_many_uneven_samples():
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("precondition", [0, 1])
 @pytest.mark.parametrize("sizes", [[((1, 2, 3), 2)], [((1, 1, 1), 1), ((9, 33, 31), 4), ((4, 8, 32), 3), ((33, 7, 5), 2), ((3, 9, 65), 1)]])
-def test_batch_in_voxel_modes_equals_general_pass(tmp_path, sizes, precision, precondition):
-    """One matrix off an isotropic one by 1e-10 sends the whole batch to the passes for any matrices
-    (C ABI): the moments differ by that and by what two solves to 1e-10 differ."""
+def test_batch_of_isotropic_materials_equals_any_matrices(tmp_path, sizes, precision, precondition):
+    """One matrix off an isotropic one by 1e-10 sends the whole batch to the diagonal of any
+    matrices (C ABI): the moments differ by that and by what two solves to 1e-10 differ."""
     import ctypes
     from chfem_b200 import _native
     from tests.test_gpu_parity import build_small, host_arrays
