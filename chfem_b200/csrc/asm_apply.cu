@@ -1,6 +1,7 @@
 // asm_apply.cu -- launches of the assembled-stencil block operator (stencil_asm.cuh) for every
 // (dof per node, precision, block size) the block solver runs.
 #include "asm_apply.h"
+#include "device_cfg.h"
 #include "stencil_asm.cuh"
 
 namespace chfem {
@@ -19,12 +20,9 @@ size_t asm_smem() { return asm_smem_bytes<ND, T, NR, ASM_TC, ND == 1 ? 2 : 1>();
 template <int ND, typename T, int NR>
 int asm_block_ctas(int R, int C, int L, int num_sms) {
   const size_t smem = asm_smem<ND, T, NR>();
-  static int per_sm = 0;  // per instantiation: the attribute is set and the occupancy asked once
-  if (!per_sm) {
-    if (cudaFuncSetAttribute(asm_kernel<ND, T, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, asm_kernel<ND, T, NR>, TE_TR * ASM_TC, smem) != cudaSuccess || per_sm < 1)
-      per_sm = 1;
-  }
+  static PerDevice kept;
+  const int per_sm = ctas_per_sm(kept, asm_kernel<ND, T, NR>, TE_TR * ASM_TC, smem);
+  if (!per_sm) return 0;
   const long work = (long)((R + TE_TR - 1) / TE_TR) * ((C + ASM_TC - 1) / ASM_TC) * L;
   return (int)std::max(1L, std::min((long)per_sm * num_sms, work / TE_MIN_RUN));
 }
@@ -37,13 +35,9 @@ cudaError_t asm_block_launch(const BlkArgs<ND, T>& a, const T* tab, int nb, cuda
 
 template <int ND, typename T, int MODE>
 int asm_te_ctas(int R, int C, int L, int num_sms) {
-  static int per_sm = 0;
-  const size_t smem = te_asm_smem_bytes<ND, T>();
-  if (!per_sm) {
-    if (cudaFuncSetAttribute(k_te_apply<ND, T, MODE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_te_apply<ND, T, MODE, true>, TE_NT, smem) != cudaSuccess || per_sm < 1)
-      per_sm = 1;
-  }
+  static PerDevice kept;
+  const int per_sm = ctas_per_sm(kept, k_te_apply<ND, T, MODE, true>, TE_NT, te_asm_smem_bytes<ND, T>());
+  if (!per_sm) return 0;
   const long work = (long)((R + TE_TR - 1) / TE_TR) * ((C + TE_TC - 1) / TE_TC) * L;
   return (int)std::max(1L, std::min((long)per_sm * num_sms, work / TE_MIN_RUN));
 }

@@ -16,6 +16,7 @@
 #include "../../include/cudapcg_b200.h"
 #include "batch_thermal.cuh"
 #include "loadcase.cuh"
+#include "device_cfg.h"
 #include "devpool.h"
 #include "modal_apply.h"
 
@@ -92,12 +93,7 @@ struct DevBuf {
   ~DevBuf() { for (void* p : ptrs) cudaFreeAsync(p, 0); }
 };
 
-int num_sms() {
-  int dev = 0, n = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n;
-}
+int num_sms() { return device_sms(); }
 template <typename K>
 int resident_ctas(K kernel, int threads) {
   int per_sm = 0;

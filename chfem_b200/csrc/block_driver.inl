@@ -52,16 +52,6 @@ static bool block_alloc(int nr) {
   return true;
 }
 
-template <int ND, typename T, int NR>
-static bool blk_prepare() {
-  static bool done = false;
-  if (!done) {
-    CKV(cudaFuncSetAttribute(k_blk_apply<ND, T, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)blk_smem_bytes<ND, T, NR>()));
-    done = true;
-  }
-  return true;
-}
-
 // The assembled-stencil block operator pass (stencil_asm.cuh, launched from asm_apply.cu), on
 // the NR right-hand sides from k0 on (dold / dnew: the direction buffers of right-hand side 0).
 template <int ND, typename T, int NR>
@@ -100,8 +90,10 @@ static bool launch_blk_apply(int parity, bool plain = false, int k0 = 0) {
   }
   if (asm_applies()) return launch_asm_block<ND, T, NR>(dold, dnew, precond, k0);
   const dim3 block(TE_TR, TE_TC);
-  if (!blk_prepare<ND, T, NR>()) return false;
-  const int nb = te_ctas(k_blk_apply<ND, T, NR>, blk_smem_bytes<ND, T, NR>());
+  static PerDevice kept;
+  const int per_sm = ctas_per_sm(kept, k_blk_apply<ND, T, NR>, TE_NT, blk_smem_bytes<ND, T, NR>());
+  if (!per_sm) { set_err("block operator", "launch configuration"); return false; }
+  const int nb = (int)std::max(1L, std::min((long)per_sm * num_sms(), te_work() / TE_MIN_RUN));
   if (!ensure_reduction(nb)) return false;
   const size_t off = (size_t)k0 * n;
   BlkArgs<ND, T> a{(const T*)B->r + off, dold + off, dnew + off, (T*)B->q + off, S->d_keys, Kdev<T>(), S->nmat, S->R, S->C, S->L, n,

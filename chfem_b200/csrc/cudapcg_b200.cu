@@ -24,6 +24,7 @@
 #include "stencil_block.cuh"
 #include "stencil_asm.cuh"
 #include "asm_apply.h"
+#include "device_cfg.h"
 #include "devpool.h"
 #include "modal_apply.h"
 #include "modal_point.cuh"
@@ -59,16 +60,7 @@ static void set_err(const char* where, const char* what) {
     if (e_ != cudaSuccess) { set_err(#call, cudaGetErrorString(e_)); return false; } \
   } while (0)
 
-static int g_num_sms = 0;
-static int num_sms() {
-  if (!g_num_sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g_num_sms <= 0) g_num_sms = 148;
-  }
-  return g_num_sms;
-}
+static int num_sms() { return device_sms(); }
 
 // ---------------------------------------------------------------------------------------
 // Dense element matrices from the reference's local-matrix formats (cudapcgSetLclMtxs).
@@ -304,7 +296,7 @@ static bool ensure_vectors() {
   S->vec_layout = layout;
   if (S->rhs_set && S->b64) {  // re-derive the working right-hand side from its FP64 copy
     if (sizeof(T) == 8) CKV(cudaMemcpyAsync(S->r, S->b64, n * 8, cudaMemcpyDeviceToDevice, S->stream));
-    else k_convert<double, float><<<std::max<long>(1, std::min<long>((n + 255) / 256, 8 * 148)), 256, 0, S->stream>>>(S->b64, (float*)S->r, (long)n);
+    else k_convert<double, float><<<std::max<long>(1, std::min<long>((n + 255) / 256, 8L * num_sms())), 256, 0, S->stream>>>(S->b64, (float*)S->r, (long)n);
   }
   if (!want_b64 && S->b64) { CKV(cudaStreamSynchronize(S->stream)); free_ptr(S->b64); S->b64 = nullptr; }
   if (p == CHFEM_B200_MIXED && !ensure_scratch64(S->y64)) return false;  // residual replacement

@@ -28,6 +28,8 @@
 #include <cstdint>
 #include <string>
 
+#include "device_cfg.h"
+
 namespace {
 
 std::string g_err;
@@ -368,12 +370,7 @@ int conv_tiles(int D, int H, int W, int planes) { return ((W + TX - 1) / TX) * (
 // Positions along H per thread (planes per tile) of k_conv: the most that still gives every SM a
 // CTA, since fewer read each weight more often.
 int conv_planes(int N, int D, int H, int W, int Cout) {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) v = 148;
-    sms = v;
-  }
+  const int sms = chfem::device_sms();
   const long per = (long)((Cout + CO_T - 1) / CO_T) * N;
   for (int p = 8; p > 2; p /= 2)
     if (conv_tiles(D, H, W, p) * per >= sms) return p;
@@ -424,13 +421,9 @@ int chfemB200NnConv3dBackwardWeight(const float* in, long in_ns, int N, int Cin,
   if (!in || !grad_out || !dw || (ksize != 1 && ksize != 3)) { g_err = "chfemB200NnConv3dBackwardWeight: bad arguments"; return 0; }
   const dim3 g(conv_tiles(D, H, W, WG_TZ), ((Cout + CO_T - 1) / CO_T) * ((Cin + WG_CI - 1) / WG_CI), N);
   const size_t smem = (size_t)(WG_CI * WG_PI + WG_TP * WG_PG) * sizeof(float);
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(k_conv_wgrad<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaFuncSetAttribute(k_conv_wgrad<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      g_err = "chfemB200NnConv3dBackwardWeight: shared-memory attribute refused"; return 0;
-    }
-    attr = true;
+  static chfem::PerDevice kept3, kept1;
+  if (!(ksize == 3 ? chfem::ctas_per_sm(kept3, k_conv_wgrad<3>, NTH, smem) : chfem::ctas_per_sm(kept1, k_conv_wgrad<1>, NTH, smem))) {
+    g_err = "chfemB200NnConv3dBackwardWeight: shared-memory attribute refused"; return 0;
   }
   if (ksize == 3) k_conv_wgrad<3><<<g, NTH, smem, (cudaStream_t)stream>>>(in, in_ns, Cin, D, H, W, grad_out, g_ns, Cout, dw, db);
   else k_conv_wgrad<1><<<g, NTH, smem, (cudaStream_t)stream>>>(in, in_ns, Cin, D, H, W, grad_out, g_ns, Cout, dw, db);

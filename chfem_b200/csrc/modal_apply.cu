@@ -4,6 +4,7 @@
 #include <cmath>
 #include <vector>
 #include "modal_apply.h"
+#include "device_cfg.h"
 #include "stencil_modal.cuh"
 #include "modal_point.cuh"
 
@@ -105,13 +106,9 @@ constexpr auto md_kernel = k_modal_apply<ND, V, MODE, md_minb<ND, V>, BLK, DENS>
 template <int ND, typename V, int MODE, bool BLK, bool DENS>
 int ctas_of(int groups, int R, int C, int L, int num_sms) {
   const size_t smem = md_smem_bytes<ND, V>();
-  static int per_sm = 0;  // per instantiation: the attribute is set and the occupancy asked once
-  if (!per_sm) {
-    int n = 0;
-    if (cudaFuncSetAttribute(md_kernel<ND, V, MODE, BLK, DENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, md_kernel<ND, V, MODE, BLK, DENS>, MD_NT, smem) != cudaSuccess || n < 1) n = 1;
-    per_sm = n;
-  }
+  static PerDevice kept;
+  const int per_sm = ctas_per_sm(kept, md_kernel<ND, V, MODE, BLK, DENS>, MD_NT, smem);
+  if (!per_sm) return 0;
   const long work = (long)groups * ((R + TE_TR - 1) / TE_TR) * ((C + MD_TC - 1) / MD_TC) * L;
   const long want = std::min(work, std::max((long)num_sms, work / 8));
   return (int)std::max((long)groups, std::min((long)per_sm * num_sms, want));
