@@ -453,7 +453,7 @@ int chfemB200NnUpsample2Backward(const float* g, long g_ns, int N, int C, int D,
 }
 // loss (device double, accumulated) and grad (may be NULL) of the mean squared error
 int chfemB200NnMse(const float* pred, const float* target, long n, float* grad, double* loss, void* stream) {
-  k_mse<<<std::min(grid1(n), 8 * 148), 256, 0, (cudaStream_t)stream>>>(pred, target, n, 1.0 / (double)n, grad, loss);
+  k_mse<<<std::min(grid1(n), 8 * chfem::device_sms()), 256, 0, (cudaStream_t)stream>>>(pred, target, n, 1.0 / (double)n, grad, loss);
   return check("chfemB200NnMse") ? 1 : 0;
 }
 int chfemB200NnAdam(float* p, const float* g, float* m, float* v, long n, float lr, float b1, float b2, float eps, int step, void* stream) {
