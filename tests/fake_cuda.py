@@ -1,0 +1,131 @@
+"""A stand-in for the CUDA runtime under the built objects of libcudapcg_b200, for checks of the host
+side that need no GPU: device memory is host memory, kernels do nothing, and the stand-in keeps
+account of what the real runtime leaves to the caller:
+
+- large dynamic shared memory is granted per (device, kernel);
+- copies and fills on the legacy stream are not ordered with the solver's non-blocking stream: work
+  there that may read or overwrite them before the legacy stream was waited for, and the reverse,
+  is recorded (fake_violations).
+"""
+import os
+import shutil
+import subprocess
+
+from tests import helpers as H
+
+OBJ = os.path.join(H.ROOT, "chfem_b200", "lib", "obj")
+OBJECTS = [os.path.join(OBJ, o + ".o") for o in ("cudapcg_b200", "modal_apply", "asm_apply", "pore_maps", "batch_thermal", "learned")]
+
+SOURCE = r'''
+#include <cstddef>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <string>
+#include <utility>
+#include <vector>
+typedef void* stream_t;
+struct dim3_ { unsigned x, y, z; };
+struct range { const char* p; size_t n; };
+static int device = 0, asked = 0;
+static std::map<std::pair<int, const void*>, int> granted;  // (device, kernel) -> bytes
+static std::vector<range> legacy, queued;  // written, not waited for: on the legacy stream; by copies and fills elsewhere
+static int n_legacy = 0, live = 0;
+static std::string bad;
+static int violations = 0;
+static void violation(const char* what) { violations++; bad += std::string(what) + "\n"; }
+static bool meets(const std::vector<range>& v, const void* p, size_t n) {
+  for (const range& r : v)
+    if (r.p < (const char*)p + n && (const char*)p < r.p + r.n) return true;
+  return false;
+}
+static void on_legacy(const char* what, void* p, size_t n) {
+  if (meets(queued, p, n)) violation((std::string(what) + " over memory that the solver's stream still writes").c_str());
+  legacy.push_back({(const char*)p, n});
+  n_legacy++;
+}
+static void on_stream(const char* what, stream_t s, void* p, size_t n, const void* src, size_t ns) {
+  if (!s) { on_legacy(what, p, n); return; }
+  if (meets(legacy, p, n) || (src && meets(legacy, src, ns))) violation((std::string(what) + " on memory that the legacy stream still writes").c_str());
+  queued.push_back({(const char*)p, n});
+}
+extern "C" {
+int fake_violations() { return violations; }
+const char* fake_report() { return bad.c_str(); }
+int fake_asked() { return asked; }
+int fake_live() { return live; }  // streams, events and pinned blocks that were not destroyed
+void fake_set_device(int d) { device = d; }
+
+int cudaGetDevice(int* d) { *d = device; return 0; }
+int cudaDeviceGetAttribute(int* v, int, int d) { *v = 100 + d; return 0; }
+int cudaDeviceSynchronize() { legacy.clear(); queued.clear(); return 0; }
+int cudaDeviceGetDefaultMemPool(void** p, int) { *p = nullptr; return 0; }
+int cudaMemPoolSetAttribute(void*, int, void*) { return 0; }
+int cudaMemPoolTrimTo(void*, size_t) { return 0; }
+int cudaMemGetInfo(size_t* f, size_t* t) { *f = *t = (size_t)1 << 40; return 0; }
+const char* cudaGetErrorString(int) { return "error of the stand-in"; }
+int cudaGetLastError() { return 0; }
+int cudaPeekAtLastError() { return 0; }
+int cudaFuncSetAttribute(const void* f, int, int bytes) { asked++; granted[{device, f}] = bytes; return 0; }
+int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int, size_t smem, unsigned) {
+  auto g = granted.find({device, f});
+  if (smem > 48 * 1024 && (g == granted.end() || (size_t)g->second < smem)) { violation("occupancy of a kernel without its shared memory"); return 1; }
+  *n = 1 + device;
+  return 0;
+}
+int cudaMallocAsync(void** p, size_t n, stream_t) { *p = calloc(1, n ? n : 1); return *p ? 0 : 2; }
+int cudaFreeAsync(void*, stream_t) { return 0; }  // kept: addresses stay distinct
+int cudaHostAlloc(void** p, size_t n, unsigned) { live++; *p = calloc(1, n); return 0; }
+int cudaFreeHost(void* p) { live--; free(p); return 0; }
+int cudaMemcpy(void* d, const void* s, size_t n, int kind) { memcpy(d, s, n); if (kind != 2) on_legacy("copy", d, n); return 0; }
+int cudaMemset(void* d, int v, size_t n) { memset(d, v, n); on_legacy("fill", d, n); return 0; }
+int cudaMemcpyToSymbol(const void*, const void*, size_t, size_t, int) { n_legacy++; return 0; }
+int cudaGetSymbolAddress(void** p, const void*) { static char scratch[1 << 20]; *p = scratch; return 0; }
+int cudaMemcpyAsync(void* d, const void* s, size_t n, int kind, stream_t st) { memcpy(d, s, n); if (kind != 2) on_stream("copy", st, d, n, kind == 3 ? s : nullptr, n); return 0; }
+int cudaMemsetAsync(void* d, int v, size_t n, stream_t st) { memset(d, v, n); on_stream("fill", st, d, n, nullptr, 0); return 0; }
+int cudaStreamCreateWithFlags(stream_t* s, unsigned) { static size_t next = 0x1000; live++; *s = (void*)next++; return 0; }
+int cudaStreamDestroy(stream_t) { live--; return 0; }
+int cudaStreamSynchronize(stream_t s) { if (s) queued.clear(); else { legacy.clear(); n_legacy = 0; } return 0; }
+int cudaStreamIsCapturing(stream_t, int* c) { *c = 0; return 0; }
+int cudaStreamBeginCapture(stream_t, int) { return 0; }
+int cudaStreamEndCapture(stream_t, void** g) { *g = (void*)1; return 0; }
+int cudaGraphInstantiate(void** x, void*, unsigned long long) { *x = (void*)1; return 0; }
+int cudaGraphDestroy(void*) { return 0; }
+int cudaGraphExecDestroy(void*) { return 0; }
+int cudaGraphLaunch(void*, stream_t) { return 0; }
+int cudaEventCreate(void** e) { live++; *e = (void*)1; return 0; }
+int cudaEventDestroy(void*) { live--; return 0; }
+int cudaEventRecord(void*, stream_t) { return 0; }
+int cudaEventSynchronize(void*) { queued.clear(); return 0; }
+int cudaEventElapsedTime(float* t, void*, void*) { *t = 1.f; return 0; }
+int cudaLaunchKernel(const void* f, dim3_, dim3_, void**, size_t smem, stream_t s) {
+  auto g = granted.find({device, f});
+  if (smem > 48 * 1024 && (g == granted.end() || (size_t)g->second < smem)) { violation("launch of a kernel without its shared memory"); return 1; }
+  if (s && n_legacy) violation("launch before the legacy stream was waited for");
+  return 0;
+}
+void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterFunction(void**, const char*, char*, const char*, int, void*, void*, void*, void*, int*) {}
+void __cudaRegisterVar(void**, char*, char*, const char*, int, size_t, int, int) {}
+static dim3_ cfg_g, cfg_b; static size_t cfg_s; static stream_t cfg_t;
+unsigned __cudaPushCallConfiguration(dim3_ g, dim3_ b, size_t s, stream_t t) { cfg_g = g; cfg_b = b; cfg_s = s; cfg_t = t; return 0; }
+int __cudaPopCallConfiguration(dim3_* g, dim3_* b, size_t* s, stream_t* t) { *g = cfg_g; *b = cfg_b; *s = cfg_s; *t = cfg_t; return 0; }
+}
+'''
+
+
+def available():
+    return bool(shutil.which("g++")) and all(os.path.exists(o) for o in OBJECTS)
+
+
+def build(workdir):
+    """libcudapcg_b200 over the stand-in, as a shared library; its path."""
+    src, lib = os.path.join(str(workdir), "fake_cuda.cpp"), os.path.join(str(workdir), "libfake_cudapcg.so")
+    with open(src, "w") as f:
+        f.write(SOURCE)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-o", lib, src, *OBJECTS], check=True,
+                   capture_output=True, text=True)
+    return lib

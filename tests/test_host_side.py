@@ -1,0 +1,84 @@
+"""Host side of the solver library over a stand-in for the CUDA runtime (fake_cuda.py): launch
+settings per device, and the order of uploads with the solver's stream."""
+import os
+import pickle
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+from tests import fake_cuda
+from tests import helpers as H
+
+pytestmark = pytest.mark.skipif(not fake_cuda.available(), reason="needs g++ and the built objects")
+
+# run in a child process: the stand-in's names are the CUDA runtime's
+PREAMBLE = r'''
+import ctypes, pickle, sys
+import numpy as np
+sys.path.insert(0, sys.argv[3])
+from chfem_b200._native import setup_cudapcg_model as setup
+lib = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_LOCAL)
+lib.fake_report.restype = ctypes.c_char_p
+models = pickle.load(open(sys.argv[2], "rb"))
+P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+lib.cudapcgB200LastError.restype = ctypes.c_char_p
+lib.cudapcgSetParametricDensityField.argtypes = [ctypes.c_void_p, ctypes.c_double, ctypes.c_double]
+def apply(a):
+    x, y = np.ones(a["ndof"]), np.zeros(a["ndof"])
+    assert lib.cudapcgB200ApplyOperator(P(x), P(y)), lib.cudapcgB200LastError()
+def block(a):
+    n = {0: 3, 1: 6}[a["analysis"]]
+    v = [np.ones(a["ndof"]) for _ in range(n)]; y = [np.zeros(a["ndof"]) for _ in range(n)]
+    arr = lambda vs: (ctypes.c_void_p * n)(*[w.ctypes.data for w in vs])
+    assert lib.cudapcgB200ApplyBlockOperator(n, arr(v), arr(y)), lib.cudapcgB200LastError()
+def free_of(fault, what):
+    lines = [l for l in lib.fake_report().decode().split("\n") if fault in l]
+    assert not lines, what + ": " + "; ".join(sorted(set(lines)))
+'''
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    """The library and one model of every analysis, in the formats of the C ABI."""
+    from tests.test_gpu_parity import host_arrays
+    wd = tmp_path_factory.mktemp("fake")
+    lib = fake_cuda.build(wd)
+    rng = np.random.default_rng(1)
+    models = {}
+    for name, analysis, nmat in (("thermal", 0, 3), ("elastic", 1, 3), ("elastic2", 1, 2), ("fluid", 2, 2)):
+        img = H.small_image((6, 7, 8), nmat, seed=2) if analysis < 2 else np.where(rng.random((6, 7, 8)) < 0.8, 0, 255).astype(np.uint8)
+        models[name] = host_arrays(*H.write_small_case(str(wd), name, img, analysis))
+    # a matrix that is not isotropic: the passes assembled by neighbour
+    models["other"] = dict(models["elastic2"], lcl=models["elastic2"]["lcl"].copy())
+    K = models["other"]["lcl"].reshape(-1, 24, 24)
+    K[:, 0::3, 0::3] *= 1.2
+    pk = os.path.join(str(wd), "models.pkl")
+    pickle.dump(models, open(pk, "wb"))
+
+    def run(script):
+        p = subprocess.run([sys.executable, "-c", PREAMBLE + script, lib, pk, H.ROOT], capture_output=True, text=True, timeout=300)
+        assert p.returncode == 0, p.stdout[-2000:] + p.stderr[-2000:]
+    return run
+
+
+def test_launch_settings_hold_on_every_device(fake):
+    """Large dynamic shared memory is granted per device, and a process may solve on one device
+    after another: every operator pass opts in on each, once."""
+    fake(r'''
+asked = []
+for turn in range(2):
+    for device in (0, 3):
+        lib.fake_set_device(device)
+        before = lib.fake_asked()
+        for name in ("thermal", "elastic", "other"):
+            for precision in (0, 1):
+                setup(lib, models[name])
+                lib.cudapcgB200SetPrecision(precision)
+                apply(models[name]); block(models[name])
+                free_of("shared memory", f"{name} on device {device}")
+                lib.cudapcgEnd()
+        asked.append(lib.fake_asked() - before)
+assert asked[0] == asked[1] > 0 and asked[2:] == [0, 0], asked
+''')
