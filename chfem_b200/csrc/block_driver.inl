@@ -44,7 +44,7 @@ static bool block_alloc(int nr) {
   std::vector<void**> vs = {&B->r, &B->d0, &B->q};
   vs.push_back(S->fluid ? &B->s : &B->d1);
   if (S->fluid) CKV(dev_malloc(&B->z, fl_record_bytes(nr)));
-  for (void** v : vs) { CKV(dev_malloc(v, tot * sizeof(T))); CKV(cudaMemset(*v, 0, tot * sizeof(T))); }
+  for (void** v : vs) { CKV(dev_malloc(v, tot * sizeof(T))); CKV(cudaMemsetAsync(*v, 0, tot * sizeof(T), S->stream)); }
   CKV(dev_malloc(&B->x, tot * 8));
   CKV(dev_malloc(&B->b64, tot * 8));
   CKV(dev_malloc(&B->sc, nr * sizeof(DevScalars)));
@@ -497,7 +497,7 @@ static bool solve_block_T(int nr, const double* const* rhs, const double* const*
     }
     if (x0 && x0[k]) {
       if (x0_mode == 1) { if (!interp_into(x0[k], slice<double>(B->x, k))) return false; }
-      else CKV(cudaMemcpyAsync(slice<double>(B->x, k), x0[k], n * 8, x0_mode == 2 ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, S->stream));
+      else CKV(upload(slice<double>(B->x, k), x0[k], n * 8, x0_mode == 2 ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice));
       has_x0[k] = true;
     }
     else CKV(cudaMemsetAsync(slice<double>(B->x, k), 0, n * 8, S->stream));

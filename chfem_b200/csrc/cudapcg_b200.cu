@@ -193,6 +193,15 @@ static cudaError_t dev_free(void* p) {
   return cudaFreeAsync(p, 0);
 }
 static void free_ptr(void* p) { dev_free(p); }
+// Uploads are made on the legacy stream, after the caller's own work on it.  The solver's
+// non-blocking stream is not ordered with it, so what is queued there is waited for first, and the
+// upload itself after: cudaMemcpy may return before a copy from pageable memory, and does before one
+// between device blocks, is complete.
+static cudaError_t legacy_wait(cudaError_t e) { return e == cudaSuccess ? cudaStreamSynchronize(0) : e; }
+static cudaError_t upload(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind = cudaMemcpyHostToDevice) {
+  const cudaError_t e = cudaStreamSynchronize(S->stream);
+  return e == cudaSuccess ? legacy_wait(cudaMemcpy(dst, src, bytes, kind)) : e;
+}
 
 static void block_invalidate();
 static void block_free();
@@ -328,7 +337,7 @@ static bool ensure_tab() {
   std::vector<T> t(t64.begin(), t64.end());
   T* d = nullptr;
   CKV(dev_malloc(&d, t.size() * sizeof(T)));
-  CKV(cudaMemcpy(d, t.data(), t.size() * sizeof(T), cudaMemcpyHostToDevice));
+  CKV(upload(d, t.data(), t.size() * sizeof(T)));
   tabdev<T>() = d;
   return true;
 }
@@ -358,7 +367,7 @@ static bool ensure_md() {
   std::vector<T> t(t64.begin(), t64.end());
   T* d = nullptr;
   CKV(dev_malloc(&d, t.size() * sizeof(T)));
-  CKV(cudaMemcpy(d, t.data(), t.size() * sizeof(T), cudaMemcpyHostToDevice));
+  CKV(upload(d, t.data(), t.size() * sizeof(T)));
   mddev<T>() = d;
   return true;
 }
@@ -429,12 +438,12 @@ static bool ensure_K() {
   for (size_t i = 0; i < kt.size(); i++) kt[i] = (T)S->Kd[i];
   T* dk = nullptr;
   CKV(dev_malloc(&dk, kt.size() * sizeof(T)));
-  CKV(cudaMemcpy(dk, kt.data(), kt.size() * sizeof(T), cudaMemcpyHostToDevice));
+  CKV(upload(dk, kt.data(), kt.size() * sizeof(T)));
   if (sizeof(T) == 8) S->d_K64 = (double*)dk; else S->d_K32 = (float*)dk;
   if (md_applies() && !ensure_md<T>()) return false;
   if (asm_applies() && !ensure_tab<T>()) return false;
   if ((S->d_sdf || S->dim2) && !ensure_invd()) return false;
-  if (S->fluid && sizeof(T) == 8) CKV(cudaMemcpyToSymbol(c_flK64, kt.data(), kt.size() * sizeof(double)));
+  if (S->fluid && sizeof(T) == 8) CKV(legacy_wait(cudaMemcpyToSymbol(c_flK64, kt.data(), kt.size() * sizeof(double))));
   return true;
 }
 
@@ -442,7 +451,7 @@ static bool ensure_K64_only() {
   if (S->d_K64) return true;
   if (!S->have_K) { set_err("solve", "local matrices were not set (cudapcgSetLclMtxs)"); return false; }
   CKV(dev_malloc(&S->d_K64, S->Kd.size() * sizeof(double)));
-  CKV(cudaMemcpy(S->d_K64, S->Kd.data(), S->Kd.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CKV(upload(S->d_K64, S->Kd.data(), S->Kd.size() * sizeof(double)));
   return true;
 }
 
@@ -1011,7 +1020,7 @@ cudapcgFlag_t cudapcgInit(cudapcgFlag_t analysis_flag, cudapcgFlag_t parStrategy
   CK(dev_malloc(&S->d_sc, sizeof(DevScalars)));
   S->cur_sc = S->d_sc;
   CK(dev_malloc(&S->d_ticket, sizeof(unsigned)));
-  CK(cudaMemset(S->d_ticket, 0, sizeof(unsigned)));
+  CK(cudaMemsetAsync(S->d_ticket, 0, sizeof(unsigned), S->stream));
   memset(S->h_sc, 0, sizeof(DevScalars));
   return CUDAPCG_TRUE;
 }
@@ -1138,12 +1147,8 @@ static bool upload_vec(const double* host, void* dst_T) {
   return true;
 }
 
-// A vector of nvars doubles into a buffer that was zeroed on the solver's stream, after that
-// zeroing (the legacy stream, on which the copy follows the caller's own work, does not wait for
-// the solver's).
 static bool copy_in(double* dst, const double* src, cudaMemcpyKind kind) {
-  CKV(cudaStreamSynchronize(S->stream));
-  CKV(cudaMemcpy(dst, src, (size_t)S->nvars * 8, kind));
+  CKV(upload(dst, src, (size_t)S->nvars * 8, kind));
   return true;
 }
 
@@ -1236,7 +1241,7 @@ cudapcgFlag_t cudapcgSetX0(cudapcgVar_t* x0, cudapcgFlag_t mustInterpolate) {
   if (!x0) {  // cudapcg.cu:298-309
     if (!S->x0_set) return CUDAPCG_TRUE;
     S->x0_set = false;
-    if (S->x) CK(cudaMemset(S->x, 0, S->nvars * 8));
+    if (S->x) CK(cudaMemsetAsync(S->x, 0, S->nvars * 8, S->stream));
     return CUDAPCG_TRUE;
   }
   if (!ensure_vectors_current()) return CUDAPCG_FALSE;
@@ -1300,13 +1305,13 @@ cudapcgFlag_t cudapcgSetImage(cudapcgMap_t* img) {
   if (S->par == CUDAPCG_EBE) {
     uint16_t* tmp = nullptr;
     CK(dev_malloc(&tmp, sizeof(uint16_t) * S->N));
-    CK(cudaMemcpy(tmp, img, sizeof(uint16_t) * S->N, cudaMemcpyHostToDevice));
+    CK(upload(tmp, img, sizeof(uint16_t) * S->N));
     if (S->dim2) k_keys_from_elements_2d<<<pw_grid(S->N), PW_NT, 0, S->stream>>>(tmp, S->d_keys, S->R, S->C);
     else k_keys_from_elements<<<pw_grid(S->N), PW_NT, 0, S->stream>>>(tmp, S->d_keys, S->R, S->C, S->L);
     CK(cudaStreamSynchronize(S->stream));
     dev_free(tmp);
   } else {
-    CK(cudaMemcpy(S->d_keys, img, sizeof(uint16_t) * S->N, cudaMemcpyHostToDevice));
+    CK(upload(S->d_keys, img, sizeof(uint16_t) * S->N));
   }
   S->have_keys = true;
   if (S->dim2) { free_ptr(S->d_invd); S->d_invd = nullptr; invalidate_graphs(); }  // a 2D Jacobi diagonal follows the keys
@@ -1425,11 +1430,11 @@ cudapcgFlag_t cudapcgSetParametricDensityField(parametricScalarField_t* field, d
   if (!S || !S->model || !field) { set_err(who, "bad arguments"); return CUDAPCG_FALSE; }
   if (S->fluid) { set_err(who, "not used for FLUID analysis"); return CUDAPCG_FALSE; }
   if (!S->d_sdf) CK(dev_malloc(&S->d_sdf, sizeof(uint16_t) * S->N));
-  CK(cudaMemcpy(S->d_sdf, field, sizeof(uint16_t) * S->N, cudaMemcpyHostToDevice));
+  CK(upload(S->d_sdf, field, sizeof(uint16_t) * S->N));
   S->sdf_min = fmin;
   S->sdf_max = fmax;
   if (!S->have_keys) {
-    CK(cudaMemset(S->d_keys, 0, sizeof(uint16_t) * S->N));
+    CK(cudaMemsetAsync(S->d_keys, 0, sizeof(uint16_t) * S->N, S->stream));
     S->have_keys = true;
   }
   free_ptr(S->d_invd); S->d_invd = nullptr;
@@ -1470,23 +1475,23 @@ cudapcgFlag_t cudapcgSetPoreMap(cudapcgFlag_t* pores) {
   if (!S->fluid) return CUDAPCG_FALSE;
   if (S->poremap_img) {  // one fluid key per node
     if (!S->d_img_fkeys) CK(dev_malloc(&S->d_img_fkeys, S->N));
-    CK(cudaMemcpy(S->d_img_fkeys, pores, S->N, cudaMemcpyHostToDevice));
+    CK(upload(S->d_img_fkeys, pores, S->N));
     S->have_img_keys = true;
     return maps_from_pore_image() ? CUDAPCG_TRUE : CUDAPCG_FALSE;
   }
-  if (S->nB) CK(cudaMemcpy(S->d_bkeys, pores, S->nB, cudaMemcpyHostToDevice));
+  if (S->nB) CK(upload(S->d_bkeys, pores, S->nB));
   return CUDAPCG_TRUE;
 }
 cudapcgFlag_t cudapcgSetPeriodic2DOFMap(cudapcgIdMap_t* vars) {
   if (!S || !S->model || !vars || !S->fluid) return CUDAPCG_FALSE;
-  CK(cudaMemcpy(S->d_dof_of_node, vars, sizeof(uint32_t) * S->N, cudaMemcpyHostToDevice));
+  CK(upload(S->d_dof_of_node, vars, sizeof(uint32_t) * S->N));
   S->have_maps = true;
   return maps_from_pore_image() ? CUDAPCG_TRUE : CUDAPCG_FALSE;
 }
 cudapcgFlag_t cudapcgSetDOF2PeriodicMap(cudapcgIdMap_t* nodes) {
   if (!S || !S->model || !nodes || !S->fluid) return CUDAPCG_FALSE;
   if (S->poremap_img) { set_err("cudapcgSetDOF2PeriodicMap", "not used with the image pore map"); return CUDAPCG_FALSE; }  // cudapcg.cu:360
-  CK(cudaMemcpy(S->d_node_of_dof, nodes, sizeof(uint32_t) * (S->nV + S->nB), cudaMemcpyHostToDevice));
+  CK(upload(S->d_node_of_dof, nodes, sizeof(uint32_t) * (S->nV + S->nB)));
   return CUDAPCG_TRUE;
 }
 
@@ -1508,8 +1513,8 @@ static bool set_fluid_diag() {
     for (int e = 0; e < NE; e++) sum -= K[(PC + e) * (ED + 1)] * (double)((k >> e) & 1);
     dg.border[k] = (sum != 0.0) ? 1.0 / sum : 0.0;
   }
-  CKV(cudaMemcpyToSymbol(c_fldiag, &dg, sizeof(FlDiag)));
-  CKV(cudaMemcpyToSymbol(d_flborder, dg.border, sizeof(dg.border)));
+  CKV(legacy_wait(cudaMemcpyToSymbol(c_fldiag, &dg, sizeof(FlDiag))));
+  CKV(legacy_wait(cudaMemcpyToSymbol(d_flborder, dg.border, sizeof(dg.border))));
   // rows of a pore node summed by neighbour (stencil_fluid_mr.cuh), [K G; G^T -Stab]
   double A[27 * 16] = {0.0};
   for (int e = 0; e < NE; e++)
@@ -1523,7 +1528,7 @@ static bool set_fluid_diag() {
       }
       blk[D * (D + 1) + D] -= K[(PC + e) * ED + PC + b];
     }
-  CKV(cudaMemcpyToSymbol(c_flA, A, sizeof(A)));
+  CKV(legacy_wait(cudaMemcpyToSymbol(c_flA, A, sizeof(A))));
   return true;
 }
 

@@ -154,7 +154,8 @@ cudapcgFlag_t cudapcgB200ApplyPreconditioner(const double *x, double *y);
    elastic; CG/PCG): rhs[k], x_out[k] are host buffers of nvars doubles, x0 may be NULL or hold
    NULL entries; x0_interpolate: 0 each x0[k] is a host vector of nvars doubles, 1 a host
    solution on the model coarsened by 2 per axis, prolonged as cudapcgSetX0(x0, 1) does, 2 a
-   device vector of nvars doubles.  Each right-hand side runs the
+   device vector of nvars doubles (read after the work that the caller queued on the legacy
+   default stream).  Each right-hand side runs the
    recurrence and stopping test of cudapcgSolve; the operator reads the model once per block
    apply.  iterations/residuals (nrhs entries) may be NULL.  Returns 1 when every right-hand
    side met the tolerance. */
@@ -250,7 +251,8 @@ cudapcgFlag_t cudapcgB200SetPoreImageColors(const uint8_t *colors, unsigned int 
    key (nbordernodes) maps copied to host buffers (any may be NULL); for tests. */
 cudapcgFlag_t cudapcgB200GetPoreMaps(uint32_t *dof_of_node, uint32_t *node_of_dof, uint8_t *border_keys);
 /* Initial guess of the next cudapcgSolve from a device vector of nvars doubles (the device
-   counterpart of cudapcgSetX0(x0, 0); cleared by cudapcgSetX0(NULL, 0)). */
+   counterpart of cudapcgSetX0(x0, 0); cleared by cudapcgSetX0(NULL, 0)).  It is read after the
+   work that the caller queued on the legacy default stream, and in full before the return. */
 cudapcgFlag_t cudapcgB200SetX0Device(const double *x0);
 /* Statistics of the last solve. */
 typedef struct {

@@ -3,9 +3,10 @@ side that need no GPU: device memory is host memory, kernels do nothing, and the
 account of what the real runtime leaves to the caller:
 
 - large dynamic shared memory is granted per (device, kernel);
+- a solve ends with the first scalar record that is read back after a graph launch (fake_finish);
 - copies and fills on the legacy stream are not ordered with the solver's non-blocking stream: work
   there that may read or overwrite them before the legacy stream was waited for, and the reverse,
-  is recorded (fake_violations).
+  is recorded (fake_report).
 """
 import os
 import shutil
@@ -32,9 +33,11 @@ static int device = 0, asked = 0;
 static std::map<std::pair<int, const void*>, int> granted;  // (device, kernel) -> bytes
 static std::vector<range> legacy, queued;  // written, not waited for: on the legacy stream; by copies and fills elsewhere
 static int n_legacy = 0, live = 0;
+static std::vector<range> pinned;
+static size_t rec_size = 0, rec_done = 0;
+static int graphs = 0, launched = 0;
 static std::string bad;
-static int violations = 0;
-static void violation(const char* what) { violations++; bad += std::string(what) + "\n"; }
+static void violation(const char* what) { bad += std::string(what) + "\n"; }
 static bool meets(const std::vector<range>& v, const void* p, size_t n) {
   for (const range& r : v)
     if (r.p < (const char*)p + n && (const char*)p < r.p + r.n) return true;
@@ -51,7 +54,8 @@ static void on_stream(const char* what, stream_t s, void* p, size_t n, const voi
   queued.push_back({(const char*)p, n});
 }
 extern "C" {
-int fake_violations() { return violations; }
+void fake_finish(size_t size, size_t done) { rec_size = size; rec_done = done; }  // a record's bytes, its flag's offset
+int fake_graphs() { return graphs; }  // captures so far
 const char* fake_report() { return bad.c_str(); }
 int fake_asked() { return asked; }
 int fake_live() { return live; }  // streams, events and pinned blocks that were not destroyed
@@ -76,24 +80,34 @@ int cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f
 }
 int cudaMallocAsync(void** p, size_t n, stream_t) { *p = calloc(1, n ? n : 1); return *p ? 0 : 2; }
 int cudaFreeAsync(void*, stream_t) { return 0; }  // kept: addresses stay distinct
-int cudaHostAlloc(void** p, size_t n, unsigned) { live++; *p = calloc(1, n); return 0; }
+int cudaHostAlloc(void** p, size_t n, unsigned) { live++; *p = calloc(1, n); pinned.push_back({(const char*)*p, n}); return 0; }
 int cudaFreeHost(void* p) { live--; free(p); return 0; }
 int cudaMemcpy(void* d, const void* s, size_t n, int kind) { memcpy(d, s, n); if (kind != 2) on_legacy("copy", d, n); return 0; }
 int cudaMemset(void* d, int v, size_t n) { memset(d, v, n); on_legacy("fill", d, n); return 0; }
 int cudaMemcpyToSymbol(const void*, const void*, size_t, size_t, int) { n_legacy++; return 0; }
 int cudaGetSymbolAddress(void** p, const void*) { static char scratch[1 << 20]; *p = scratch; return 0; }
-int cudaMemcpyAsync(void* d, const void* s, size_t n, int kind, stream_t st) { memcpy(d, s, n); if (kind != 2) on_stream("copy", st, d, n, kind == 3 ? s : nullptr, n); return 0; }
+int cudaMemcpyAsync(void* d, const void* s, size_t n, int kind, stream_t st) {
+  memcpy(d, s, n);
+  if (kind != 2) on_stream("copy", st, d, n, kind == 3 ? s : nullptr, n);
+  else if (launched && rec_size && n % rec_size == 0 && meets(pinned, d, n))
+    for (size_t k = 0; k < n; k += rec_size) { const int one = 1; memcpy((char*)d + k + rec_done, &one, sizeof(int)); }
+  return 0;
+}
 int cudaMemsetAsync(void* d, int v, size_t n, stream_t st) { memset(d, v, n); on_stream("fill", st, d, n, nullptr, 0); return 0; }
 int cudaStreamCreateWithFlags(stream_t* s, unsigned) { static size_t next = 0x1000; live++; *s = (void*)next++; return 0; }
 int cudaStreamDestroy(stream_t) { live--; return 0; }
 int cudaStreamSynchronize(stream_t s) { if (s) queued.clear(); else { legacy.clear(); n_legacy = 0; } return 0; }
 int cudaStreamIsCapturing(stream_t, int* c) { *c = 0; return 0; }
-int cudaStreamBeginCapture(stream_t, int) { return 0; }
+int cudaStreamBeginCapture(stream_t, int) { graphs++; return 0; }
 int cudaStreamEndCapture(stream_t, void** g) { *g = (void*)1; return 0; }
 int cudaGraphInstantiate(void** x, void*, unsigned long long) { *x = (void*)1; return 0; }
 int cudaGraphDestroy(void*) { return 0; }
 int cudaGraphExecDestroy(void*) { return 0; }
-int cudaGraphLaunch(void*, stream_t) { return 0; }
+int cudaGraphLaunch(void*, stream_t s) {
+  if (s && n_legacy) violation("launch before the legacy stream was waited for");
+  launched = 1;
+  return 0;
+}
 int cudaEventCreate(void** e) { live++; *e = (void*)1; return 0; }
 int cudaEventDestroy(void*) { live--; return 0; }
 int cudaEventRecord(void*, stream_t) { return 0; }

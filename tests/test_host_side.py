@@ -33,8 +33,19 @@ def block(a):
     v = [np.ones(a["ndof"]) for _ in range(n)]; y = [np.zeros(a["ndof"]) for _ in range(n)]
     arr = lambda vs: (ctypes.c_void_p * n)(*[w.ctypes.data for w in vs])
     assert lib.cudapcgB200ApplyBlockOperator(n, arr(v), arr(y)), lib.cudapcgB200LastError()
+class Scalars(ctypes.Structure):  # DevScalars (common.cuh)
+    _fields_ = [(n, ctypes.c_double) for n in "delta delta0 delta_old alpha beta res0 metric".split()] + [
+        ("red", ctypes.c_double * 6), ("xa", ctypes.c_double)] + [(n, ctypes.c_int) for n in "iteration done found status".split()]
+lib.fake_finish(ctypes.c_size_t(ctypes.sizeof(Scalars)), ctypes.c_size_t(Scalars.done.offset))
+lib.cudapcgSetNumTol.argtypes = [ctypes.c_double]
+def solve(a):
+    x = np.zeros(a["ndof"])
+    lib.cudapcgSolve(P(x))
+    assert not lib.cudapcgB200LastError(), lib.cudapcgB200LastError()
+def rhs(a):
+    assert lib.cudapcgSetRHS(P(np.ones(a["ndof"]))), lib.cudapcgB200LastError()
 def free_of(fault, what):
-    lines = [l for l in lib.fake_report().decode().split("\n") if fault in l]
+    lines = [l for l in lib.fake_report().decode().split("\n") if l and fault in l]
     assert not lines, what + ": " + "; ".join(sorted(set(lines)))
 '''
 
@@ -81,4 +92,48 @@ for turn in range(2):
                 lib.cudapcgEnd()
         asked.append(lib.fake_asked() - before)
 assert asked[0] == asked[1] > 0 and asked[2:] == [0, 0], asked
+''')
+
+
+def test_uploads_and_passes_are_ordered(fake):
+    """Whatever is uploaded on the legacy stream is in place before a pass on the solver's stream, and
+    no upload meets a fill that is still queued there -- for every entry point that takes model data,
+    also on a model whose vectors exist already (no allocation in between)."""
+    fake(r'''
+for name in ("thermal", "elastic", "other", "fluid"):
+    a = models[name]
+    fluid = name == "fluid"
+    for precision in (0, 1):
+        setup(lib, a)
+        lib.cudapcgB200SetPrecision(precision)
+        lib.cudapcgSetSolver(1 if fluid else 0)
+        apply(a); rhs(a); solve(a)
+        free_of("", name)
+        guess = np.ones(a["ndof"])
+        keep = [np.ascontiguousarray(a[k]) for k in ("keys", "dof_of_node", "border", "node_of_dof", "lcl")]
+        steps = [lambda: lib.cudapcgSetX0(P(guess), 0), lambda: lib.cudapcgB200SetX0Device(P(guess)), lambda: lib.cudapcgSetX0(None, 0),
+                 lambda: lib.cudapcgSetX0(P(guess), 0), lambda: lib.cudapcgSetLclMtxs(P(keep[4]))]
+        if fluid:
+            steps += [lambda: lib.cudapcgSetPeriodic2DOFMap(P(keep[1])), lambda: lib.cudapcgSetPoreMap(P(keep[2])),
+                      lambda: lib.cudapcgSetDOF2PeriodicMap(P(keep[3]))]
+        else:
+            density = np.full(a["N"], 7, np.uint16)
+            steps += [lambda: lib.cudapcgSetImage(P(keep[0])), lambda: lib.cudapcgSetParametricDensityField(P(density), 0.5, 1.5),
+                      lambda: lib.cudapcgSetImage(P(keep[0]))]
+        for i, step in enumerate(steps):
+            assert step(), (i, lib.cudapcgB200LastError())
+            rhs(a); solve(a)
+            free_of("", f"{name}, precision {precision}, step {i}")
+        lib.cudapcgEnd()
+        n = 6 if name in ("elastic", "other") else 3
+        arr = lambda vs: (ctypes.c_void_p * n)(*[v.ctypes.data for v in vs])
+        b, x, g = ([np.ones(a["ndof"]) for _ in range(n)] for _ in range(3))
+        setup(lib, a)
+        lib.cudapcgB200SetPrecision(precision)
+        lib.cudapcgSetSolver(1 if fluid else 0)
+        for mode in (0, 2, 0, 2):
+            lib.cudapcgB200SolveBlock(n, arr(b), arr(g), mode, arr(x), None, None)
+            assert not lib.cudapcgB200LastError(), lib.cudapcgB200LastError()
+            free_of("", f"{name} block, precision {precision}, guess {mode}")
+        lib.cudapcgEnd()
 ''')
