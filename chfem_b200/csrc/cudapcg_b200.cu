@@ -1086,8 +1086,19 @@ cudapcgFlag_t cudapcgBuildModel(const void* data) {
   return adopt_model();
 }
 
-cudapcgFlag_t cudapcgSetNumTol(cudapcgTol_t t) { if (!S) return CUDAPCG_FALSE; S->tol = t; return CUDAPCG_TRUE; }
-cudapcgFlag_t cudapcgSetMaxIterations(unsigned int n) { if (!S) return CUDAPCG_FALSE; S->maxit = n; return CUDAPCG_TRUE; }
+// the captured passes hold the tolerance and the iteration limit
+cudapcgFlag_t cudapcgSetNumTol(cudapcgTol_t t) {
+  if (!S) return CUDAPCG_FALSE;
+  if (!(t == S->tol)) invalidate_graphs();
+  S->tol = t;
+  return CUDAPCG_TRUE;
+}
+cudapcgFlag_t cudapcgSetMaxIterations(unsigned int n) {
+  if (!S) return CUDAPCG_FALSE;
+  if (n != S->maxit) invalidate_graphs();
+  S->maxit = n;
+  return CUDAPCG_TRUE;
+}
 cudapcgFlag_t cudapcgSetXReduceMode(cudapcgFlag_t flag) {
   if (!S) return CUDAPCG_FALSE;
   S->xr_mode = flag <= CUDAPCG_XREDUCE_FULL ? flag : CUDAPCG_XREDUCE_FULL;

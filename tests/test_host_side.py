@@ -137,3 +137,36 @@ for name in ("thermal", "elastic", "other", "fluid"):
             free_of("", f"{name} block, precision {precision}, guess {mode}")
         lib.cudapcgEnd()
 ''')
+
+
+def test_captured_passes_follow_the_settings(fake):
+    """A graph of passes captured for one tolerance, iteration limit, norm, preconditioner or solver
+    is not replayed under another; the same settings replay it."""
+    fake(r'''
+lib.cudapcgSetMaxIterations.argtypes = [ctypes.c_uint]
+for name in ("thermal", "elastic", "fluid"):
+    a = models[name]
+    minres = 1 if name == "fluid" else 0
+    n = 6 if name == "elastic" else 3
+    arr = lambda vs: (ctypes.c_void_p * n)(*[v.ctypes.data for v in vs])
+    b, x = [np.ones(a["ndof"]) for _ in range(n)], [np.zeros(a["ndof"]) for _ in range(n)]
+    def solve_block(a):
+        lib.cudapcgB200SolveBlock(n, arr(b), None, 0, arr(x), None, None)
+        assert not lib.cudapcgB200LastError(), lib.cudapcgB200LastError()
+    solvers = [(minres, solve), (minres, solve_block)] + ([(5, solve)] if minres else [(2, solve), (1, solve)])
+    for solver, run in solvers:
+        setup(lib, a)
+        lib.cudapcgSetSolver(solver)
+        def captures():
+            before = lib.fake_graphs()
+            if run is solve: rhs(a)
+            run(a)
+            return lib.fake_graphs() - before
+        assert captures() == 1 and captures() == 0
+        for change in (lambda: lib.cudapcgSetNumTol(1e-3), lambda: lib.cudapcgSetMaxIterations(77), lambda: lib.cudapcgSetResNorm(1),
+                       lambda: lib.cudapcgSetPreconditioner(0), lambda: lib.cudapcgB200SetIterationsPerLaunch(8)):
+            assert change()
+            assert captures() == 1, (name, solver)
+            assert captures() == 0, (name, solver)
+        lib.cudapcgEnd()
+''')
