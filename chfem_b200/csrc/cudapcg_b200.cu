@@ -412,6 +412,13 @@ static bool ensure_invd() {
   CKV(cudaGetLastError());
   return true;
 }
+// the precomputed diagonal (2D models, scalar density field) follows the keys
+static void drop_invd() {
+  if (!S->d_invd) return;
+  free_ptr(S->d_invd);
+  S->d_invd = nullptr;
+  invalidate_graphs();  // captured launches hold its pointer
+}
 // the scalar-density-field arguments of a thermal / elastic operator pass
 template <int ND, typename T>
 static void sdf_args(TeArgs<ND, T>& a) {
@@ -1325,7 +1332,7 @@ cudapcgFlag_t cudapcgSetImage(cudapcgMap_t* img) {
     CK(upload(S->d_keys, img, sizeof(uint16_t) * S->N));
   }
   S->have_keys = true;
-  if (S->dim2) { free_ptr(S->d_invd); S->d_invd = nullptr; invalidate_graphs(); }  // a 2D Jacobi diagonal follows the keys
+  drop_invd();
   return CUDAPCG_TRUE;
 }
 cudapcgFlag_t cudapcgB200SetImageColors(const uint8_t* colors, unsigned int rows, unsigned int cols, unsigned int slices,
@@ -1362,6 +1369,7 @@ cudapcgFlag_t cudapcgB200SetImageColors(const uint8_t* colors, unsigned int rows
   if (e != cudaSuccess) { set_err(who, cudaGetErrorString(e)); return CUDAPCG_FALSE; }
   if (bad) { set_err(who, "the image holds a colour without a material (or a material index above 3)"); return CUDAPCG_FALSE; }
   S->have_keys = true;
+  drop_invd();
   invalidate_graphs();
   return CUDAPCG_TRUE;
 }

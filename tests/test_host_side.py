@@ -170,3 +170,31 @@ for name in ("thermal", "elastic", "fluid"):
             assert captures() == 0, (name, solver)
         lib.cudapcgEnd()
 ''')
+
+
+def test_jacobi_diagonal_follows_the_image(fake):
+    """Under a density field the inverse diagonal is computed once per model from keys and density:
+    a new image on the same model drops it, and the graphs that hold its address."""
+    fake(r'''
+import tempfile
+for name in ("thermal", "elastic"):
+    a = models[name]
+    setup(lib, a)
+    density = np.full(a["N"], 7, np.uint16)
+    assert lib.cudapcgSetParametricDensityField(P(density), 0.5, 1.5)
+    keys = np.ascontiguousarray(a["keys"])
+    colors = np.zeros(a["N"], np.uint8)
+    lut = (ctypes.c_int * 256)(*([0] * 256))
+    rhs(a); solve(a)
+    for image in (lambda: lib.cudapcgSetImage(P(keys)),
+                  lambda: lib.cudapcgB200SetImageColors(P(colors), a["ny"], a["nx"], a["nz"], 1, lut)):
+        launched, graphs = lib.fake_launches(), lib.fake_graphs()
+        rhs(a); solve(a)
+        same = lib.fake_launches() - launched
+        assert lib.fake_graphs() == graphs
+        assert image(), lib.cudapcgB200LastError()
+        launched = lib.fake_launches()
+        rhs(a); solve(a)
+        assert lib.fake_launches() - launched > same and lib.fake_graphs() == graphs + 1, name
+    lib.cudapcgEnd()
+''')
