@@ -263,7 +263,8 @@ static bool ensure_scratch64(double*& p) {
 static size_t fl_record_bytes(int nr);
 
 // Work vectors for precision T, as many as the selected solver reads:
-//   every solver      x (FP64), r, the direction's two buffers d0 / d1
+//   every solver      x (FP64), r, the direction d0
+//   PCG               d1, the direction's second buffer ((P)MINRES updates the direction in place)
 //   PCG / MINRES      q = A d
 //   Stokes, MINRES    s (Stokes PCG reads a stored M^-1 r; (P)MINRES keeps A M^-1 r)
 //   MINRES            thermal, elastic: r2 (the residual's second buffer); Stokes: fl_z
@@ -292,7 +293,8 @@ static bool ensure_vectors() {
     CKV(cudaMemsetAsync(S->b64, 0, n * 8, S->stream));
   }
   free_work_vectors();
-  std::vector<void**> vs = {&S->r, &S->d0, &S->d1};
+  std::vector<void**> vs = {&S->r, &S->d0};
+  if (!minres_solver()) vs.push_back(&S->d1);
   if (!pcg3_solver()) vs.push_back(&S->q);
   if (S->fluid || minres_solver()) vs.push_back(&S->s);
   if (minres_solver() && !S->fluid) vs.push_back(&S->r2);
@@ -1647,8 +1649,9 @@ template <typename T>
 static bool apply_host_T(const double* xh, double* yh, bool precond_only) {
   if (!ensure_vectors<T>() || !ensure_K<T>()) return false;
   const size_t n = (size_t)S->nvars;
-  // the direction buffers are free between solves: d0 takes the input, d1 the output (the
-  // solver state in x and r stays untouched)
+  // the direction buffers (and q) are free between solves: d0 takes the input, the second the
+  // output (the solver state in x and r stays untouched)
+  void* const out = S->d1 ? S->d1 : S->q;
   if (!upload_vec(xh, S->d0)) return false;
   if (!ensure_reduction(8 * num_sms())) return false;
   CKV(cudaMemsetAsync(S->d_sc, 0, sizeof(DevScalars), S->stream));
@@ -1657,16 +1660,16 @@ static bool apply_host_T(const double* xh, double* yh, bool precond_only) {
     if (!ensure_scratch64(S->x64)) return false;
     CKV(cudaMemcpyAsync(S->x64, S->r, n * sizeof(T), cudaMemcpyDeviceToDevice, S->stream));
     CKV(cudaMemcpyAsync(S->r, S->d0, n * sizeof(T), cudaMemcpyDeviceToDevice, S->stream));
-    if (!launch_point<T, PW_INIT>(S->x, nullptr, (T*)S->r, nullptr, (T*)S->d1, nullptr)) return false;
+    if (!launch_point<T, PW_INIT>(S->x, nullptr, (T*)S->r, nullptr, (T*)out, nullptr)) return false;
     CKV(cudaMemcpyAsync(S->r, S->x64, n * sizeof(T), cudaMemcpyDeviceToDevice, S->stream));
   } else {
-    if (!launch_apply<T>((const T*)S->d0, nullptr, nullptr, (T*)S->d1, false, FIN_STORE, false)) return false;
+    if (!launch_apply<T>((const T*)S->d0, nullptr, nullptr, (T*)out, false, FIN_STORE, false)) return false;
   }
   if (sizeof(T) == 8) {
-    CKV(cudaMemcpyAsync(yh, S->d1, n * 8, cudaMemcpyDeviceToHost, S->stream));
+    CKV(cudaMemcpyAsync(yh, out, n * 8, cudaMemcpyDeviceToHost, S->stream));
   } else {
     if (!ensure_scratch64(S->x64)) return false;
-    k_convert<float, double><<<pw_grid(n), PW_NT, 0, S->stream>>>((const float*)S->d1, S->x64, n);
+    k_convert<float, double><<<pw_grid(n), PW_NT, 0, S->stream>>>((const float*)out, S->x64, n);
     CKV(cudaMemcpyAsync(yh, S->x64, n * 8, cudaMemcpyDeviceToHost, S->stream));
   }
   CKV(cudaStreamSynchronize(S->stream));
@@ -1701,9 +1704,10 @@ static double time_op_T(unsigned reps) {
   if (!ensure_vectors<T>() || !ensure_K<T>()) return -1.0;
   if (!ensure_reduction(8 * num_sms())) return -1.0;
   cudaMemsetAsync(S->d_sc, 0, sizeof(DevScalars), S->stream);
-  for (int w = 0; w < 3; w++) launch_apply<T>((const T*)S->d0, nullptr, nullptr, (T*)S->d1, false, FIN_NONE, false);
+  T* const out = (T*)(S->d1 ? S->d1 : S->q);
+  for (int w = 0; w < 3; w++) launch_apply<T>((const T*)S->d0, nullptr, nullptr, out, false, FIN_NONE, false);
   cudaEventRecord(S->ev0, S->stream);
-  for (unsigned i = 0; i < reps; i++) launch_apply<T>((const T*)S->d0, nullptr, nullptr, (T*)S->d1, false, FIN_NONE, false);
+  for (unsigned i = 0; i < reps; i++) launch_apply<T>((const T*)S->d0, nullptr, nullptr, out, false, FIN_NONE, false);
   cudaEventRecord(S->ev1, S->stream);
   if (cudaEventSynchronize(S->ev1) != cudaSuccess) return -1.0;
   float ms = 0;
@@ -1715,7 +1719,7 @@ extern "C" {
 template <typename T>
 static double time_kernel_T(int which, unsigned reps) {
   if (!ensure_vectors<T>() || !ensure_K<T>()) return -1.0;
-  if (!S->q || ((which == 3 || which == 4) && !S->r2 && !S->fl_z)) { set_err("cudapcgB200TimeKernel", "kernel not used by the selected solver"); return -1.0; }
+  if (!S->q || ((which == 1 || which == 2) && !S->d1) || ((which == 3 || which == 4) && !S->r2 && !S->fl_z)) { set_err("cudapcgB200TimeKernel", "kernel not used by the selected solver"); return -1.0; }
   if (!ensure_reduction(needed_blocks())) return -1.0;
   // each repetition resets the scalars (so no pass exits early) and brackets only the launch
   float total = 0.f;

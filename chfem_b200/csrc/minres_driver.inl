@@ -14,8 +14,9 @@ static MrCfg mrcfg() {
 
 // Whether the Stokes records of nr directions are kept per grid node (stencil_fluid_mr.cuh): 8 %
 // faster than per fluid node at 96^3 and porosity 0.35, for 32 N nr bytes instead of 32 (nV + nB) nr.
-// Not where the grid holds more than four nodes per fluid node or its records exceed 16 GiB, so
-// that a model that fills the device memory needs no more of it.
+// Not where the grid holds more than four nodes per fluid node (128 bytes per fluid node) or its
+// records exceed 16 GiB: what a model that fills the device holds beside its vectors, 48 bytes per
+// unknown, is then 32 bytes per fluid node.
 static bool fl_by_node(int nr) { return S->N <= 4l * (S->nV + S->nB) && 32l * S->N * nr <= 16l << 30; }
 static size_t fl_record_bytes(int nr) { return 32ul * nr * std::max(fl_by_node(nr) ? S->N : S->nV + S->nB, 1l); }
 

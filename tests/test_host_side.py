@@ -69,7 +69,8 @@ def fake(tmp_path_factory):
     pickle.dump(models, open(pk, "wb"))
 
     def run(script):
-        p = subprocess.run([sys.executable, "-c", PREAMBLE + script, lib, pk, H.ROOT], capture_output=True, text=True, timeout=300)
+        p = subprocess.run([sys.executable, "-c", PREAMBLE + script, lib, pk, H.ROOT], capture_output=True, text=True, timeout=300,
+                           cwd=str(wd))
         assert p.returncode == 0, p.stdout[-2000:] + p.stderr[-2000:]
     return run
 
@@ -197,4 +198,32 @@ for name in ("thermal", "elastic"):
         rhs(a); solve(a)
         assert lib.fake_launches() - launched > same and lib.fake_graphs() == graphs + 1, name
     lib.cudapcgEnd()
+''')
+
+
+def test_device_bytes_of_minres(fake):
+    """(P)MINRES keeps one direction buffer: x, b, r, r', d, q, s on thermal and elastic models (56 B
+    per unknown in FP64; 44 B mixed, with the FP64 scratch of the residual replacement), x, b, r,
+    d, q, s and the records of M^-1 r on Stokes models; the operator can still be applied."""
+    fake(r'''
+lib.cudapcgB200DeviceBytes.restype = ctypes.c_ulonglong
+for name in ("thermal", "elastic", "fluid"):
+    a = models[name]
+    for precision in (0, 1) if name != "fluid" else (0,):
+        setup(lib, a)
+        lib.cudapcgB200SetPrecision(precision)
+        lib.cudapcgSetSolver(1)
+        rhs(a); solve(a)
+        held = lib.cudapcgB200DeviceBytes()
+        if name == "fluid":
+            nodes = a["nV"] + a["nB"]
+            records = 32 * (a["N"] if a["N"] <= 4 * nodes else nodes)
+            assert held <= 48 * a["ndof"] + records + 4 * a["N"] + 4 * nodes + a["nB"], held / a["ndof"]
+        else:
+            assert held <= (44 if precision else 56) * a["ndof"] + 2 * a["N"], (name, precision, held / a["ndof"])
+        apply(a)
+        lib.cudapcgB200TimeOperator.restype = lib.cudapcgB200TimeKernel.restype = ctypes.c_double
+        assert lib.cudapcgB200TimeOperator(1) > 0 and lib.cudapcgB200TimeKernel(3, 1) > 0
+        free_of("", name)
+        lib.cudapcgEnd()
 ''')
