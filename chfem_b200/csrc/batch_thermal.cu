@@ -36,7 +36,8 @@ std::map<std::string, int> g_tile_cache;
 
 // The stream, its events and the pinned schedule record of a batch serve the next one on the same
 // device (as cudapcgEnd keeps a solver's: their destruction alone cost up to 0.7 s a call).  At
-// most 4 sets are kept, for as many threads; a batch that failed destroys its own.
+// most 4 sets are kept, for as many threads, until cudapcgB200TrimMemory; a batch that failed
+// destroys its own.
 struct BtHandles {
   int dev = -1;
   cudaStream_t st = nullptr;
@@ -63,6 +64,12 @@ bool take_handles(BtHandles& h) {
   BT_CK(cudaMallocHost(&h.h_sch, sizeof(BtSched)));
   return true;
 }
+void destroy_handles(BtHandles& h) {
+  if (h.h_sch) cudaFreeHost(h.h_sch);
+  for (cudaEvent_t e : h.ev)
+    if (e) cudaEventDestroy(e);
+  if (h.st) cudaStreamDestroy(h.st);
+}
 void give_handles(BtHandles& h, bool keep) {
   if (keep) {
     std::lock_guard<std::mutex> lock(g_idle_mutex);
@@ -71,10 +78,7 @@ void give_handles(BtHandles& h, bool keep) {
       return;
     }
   }
-  if (h.h_sch) cudaFreeHost(h.h_sch);
-  for (cudaEvent_t e : h.ev)
-    if (e) cudaEventDestroy(e);
-  if (h.st) cudaStreamDestroy(h.st);
+  destroy_handles(h);
 }
 
 // Device memory of a batch, from the same pool as the solver's.  The batch waits for its stream
@@ -370,6 +374,15 @@ int run_batch(const Inputs& in, bool mixed, double* moments, unsigned* iteration
 }
 
 }  // namespace
+
+void chfem::release_batch_handles() {
+  std::vector<BtHandles> idle;
+  {
+    std::lock_guard<std::mutex> lock(g_idle_mutex);
+    idle.swap(g_idle);
+  }
+  for (BtHandles& h : idle) destroy_handles(h);
+}
 
 extern "C" int cudapcgB200SolveThermalBatch(unsigned int nsamples, const unsigned int* dims, const uint16_t* const* keys,
                                             const unsigned int* nmat, const double* const* Kdense, const double* const* CB,

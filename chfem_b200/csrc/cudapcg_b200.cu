@@ -954,7 +954,8 @@ const char* cudapcgB200LastError(void) { return g_err.c_str(); }
 
 // The stream, its three events and the pinned scalar record outlive a solver: cudapcgEnd keeps
 // them for the next cudapcgInit on the same device (destroying and re-creating them cost up to
-// 0.7 s per model on some B200 boxes).  A solver on another device gets new ones.
+// 0.7 s per model on some B200 boxes), until cudapcgB200TrimMemory.  A solver on another device
+// gets new ones.
 struct KeptHandles {
   int dev = -1;
   cudaStream_t stream = nullptr;
@@ -962,19 +963,19 @@ struct KeptHandles {
   DevScalars* h_sc = nullptr;
 };
 static KeptHandles g_kept;
+static void destroy_handles(const KeptHandles& k) {
+  if (k.h_sc) cudaFreeHost(k.h_sc);
+  for (cudaEvent_t e : k.ev)
+    if (e) cudaEventDestroy(e);
+  if (k.stream) cudaStreamDestroy(k.stream);
+}
 static void keep_handles() {
   int dev = -1;
   if (S->stream) cudaStreamSynchronize(S->stream);
-  if (cudaGetDevice(&dev) == cudaSuccess && S->stream && S->ev0 && S->ev1 && S->ev2 && S->h_sc && !g_kept.stream) {
-    g_kept.dev = dev; g_kept.stream = S->stream; g_kept.ev[0] = S->ev0; g_kept.ev[1] = S->ev1; g_kept.ev[2] = S->ev2;
-    g_kept.h_sc = S->h_sc;
-    return;
-  }
-  if (S->h_sc) cudaFreeHost(S->h_sc);
-  if (S->ev0) cudaEventDestroy(S->ev0);
-  if (S->ev1) cudaEventDestroy(S->ev1);
-  if (S->ev2) cudaEventDestroy(S->ev2);
-  if (S->stream) cudaStreamDestroy(S->stream);
+  const bool have_dev = cudaGetDevice(&dev) == cudaSuccess;
+  const KeptHandles k{dev, S->stream, {S->ev0, S->ev1, S->ev2}, S->h_sc};
+  if (have_dev && k.stream && k.ev[0] && k.ev[1] && k.ev[2] && k.h_sc && !g_kept.stream) g_kept = k;
+  else destroy_handles(k);
 }
 static bool take_kept_handles() {
   int dev = -1;
@@ -1764,6 +1765,9 @@ double cudapcgB200TimeOperator(unsigned int reps) {
 int cudapcgB200TrimMemory(void) {
   int dev = 0;
   cudaMemPool_t pool;
+  release_batch_handles();
+  destroy_handles(g_kept);
+  g_kept = KeptHandles();
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = cudaDeviceGetDefaultMemPool(&pool, dev);

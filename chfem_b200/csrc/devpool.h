@@ -24,4 +24,7 @@ inline void pool_keep() {
   kept[dev] = true;
 }
 
+// Destroys the handles that finished batches keep for the next (batch_thermal.cu).
+void release_batch_handles();
+
 }  // namespace chfem

@@ -296,10 +296,13 @@ int cudapcgB200ApplyOperatorNoAlloc(int analysis_flag, unsigned int nrows, unsig
                                     double *y, double *vAv, void *stream);
 /* Number of bytes the library holds on the device for the current model and arrays. */
 unsigned long long cudapcgB200DeviceBytes(void);
-/* The solver's device blocks come from the current device's default stream-ordered memory pool,
-   which keeps freed blocks (up to a quarter of the device's memory) mapped for the next model
-   (cudapcgEnd returns them to the pool, not to the driver).  This hands every kept block of the pool back to the driver.  Returns 1, or 0
-   with cudapcgB200LastError() set. */
+/* The device blocks of a solver and of a batch (cudapcgB200SolveThermalBatch) come from the current
+   device's default stream-ordered memory pool, which keeps freed blocks mapped for the next model
+   or batch, up to a quarter of the device's memory (or CHFEM_B200_POOL_KEEP_BYTES): cudapcgEnd and
+   the end of a batch return them to the pool, not to the driver, and an allocator beside the pool
+   cannot use them.  One solver's and up to four batches' stream, events and pinned record are kept
+   likewise.  This hands every kept block of the pool back to the driver and destroys the kept
+   handles.  Returns 1, or 0 with cudapcgB200LastError() set. */
 int cudapcgB200TrimMemory(void);
 
 #ifdef __cplusplus

@@ -227,3 +227,31 @@ for name in ("thermal", "elastic", "fluid"):
         free_of("", name)
         lib.cudapcgEnd()
 ''')
+
+
+def test_trim_releases_what_is_kept(fake):
+    """A solver's and a batch's stream, events and pinned record outlive them, serve the next, and go
+    with cudapcgB200TrimMemory, as do those of batches in several threads."""
+    fake(r'''
+import threading
+lib.cudapcgB200BatchLastError.restype = ctypes.c_char_p
+a = models["thermal"]
+def batch():
+    keys, nmat, K, CB = np.ascontiguousarray(a["keys"]), np.array([a["nkeys"]], np.uint32), np.ones(256), np.ones(96)
+    one = lambda v: (ctypes.c_void_p * 1)(v.ctypes.data)
+    dims = np.array([[a["ny"], a["nx"], a["nz"]]], np.uint32)
+    m, its, res = np.zeros(9), np.zeros(3, np.uint32), np.zeros(3)
+    assert lib.cudapcgB200SolveThermalBatch(ctypes.c_uint(1), P(dims), one(keys), P(nmat), one(K), one(CB), ctypes.c_double(1e-6),
+                                            ctypes.c_uint(10), 0, 1, P(m), P(its), P(res), None), lib.cudapcgB200BatchLastError()
+for turn in range(2):
+    setup(lib, a); rhs(a); solve(a); lib.cudapcgEnd()
+    batch()
+    kept = lib.fake_live()
+    assert kept > 0
+    setup(lib, a); rhs(a); solve(a); lib.cudapcgEnd()
+    batch()
+    assert lib.fake_live() == kept
+    threads = [threading.Thread(target=batch) for _ in range(8)]
+    [t.start() for t in threads]; [t.join() for t in threads]
+    assert lib.cudapcgB200TrimMemory() and lib.fake_live() == 0, lib.fake_live()
+''')
