@@ -24,7 +24,7 @@ using namespace chfem;
 
 namespace {
 
-std::string g_err;
+thread_local std::string g_err;  // of the calling thread's last batch
 #define BT_CK(call)                                                      \
   do {                                                                   \
     cudaError_t e_ = (call);                                             \
@@ -33,6 +33,7 @@ std::string g_err;
 
 // tile width chosen per batch signature (sizes histogram, precision)
 std::map<std::string, int> g_tile_cache;
+std::mutex g_tile_mutex;
 
 // The stream, its events and the pinned schedule record of a batch serve the next one on the same
 // device (as cudapcgEnd keeps a solver's: their destruction alone cost up to 0.7 s a call).  At
@@ -359,13 +360,17 @@ int run_batch(const Inputs& in, bool mixed, double* moments, unsigned* iteration
     for (unsigned s = 0; s < in.n; s++) hist[std::to_string(in.dims[3 * s]) + "x" + std::to_string(in.dims[3 * s + 1]) + "x" + std::to_string(in.dims[3 * s + 2])]++;
     for (auto& kv : hist) sig += ":" + kv.first + "*" + std::to_string(kv.second);
   }
-  int tc;
-  auto it = g_tile_cache.find(sig);
-  if (it != g_tile_cache.end()) tc = it->second;
-  else {
+  int tc = 0;
+  {
+    std::lock_guard<std::mutex> lock(g_tile_mutex);
+    const auto it = g_tile_cache.find(sig);
+    if (it != g_tile_cache.end()) tc = it->second;
+  }
+  if (!tc) {
     const double t4 = b.template time_apply<4>(), t8 = b.template time_apply<8>(), t16 = b.template time_apply<16>();
     tc = (t4 <= t8 && t4 <= t16) ? 4 : (t8 <= t16 ? 8 : 16);
     if (stats) { stats->tile_ms[0] = t4; stats->tile_ms[1] = t8; stats->tile_ms[2] = t16; }
+    std::lock_guard<std::mutex> lock(g_tile_mutex);
     g_tile_cache[sig] = tc;
   }
   bool ok = tc == 4 ? b.template solve<4>(mixed, stats) : (tc == 8 ? b.template solve<8>(mixed, stats) : b.template solve<16>(mixed, stats));

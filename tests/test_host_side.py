@@ -255,3 +255,30 @@ for turn in range(2):
     [t.start() for t in threads]; [t.join() for t in threads]
     assert lib.cudapcgB200TrimMemory() and lib.fake_live() == 0, lib.fake_live()
 ''')
+
+
+def test_batches_in_threads_keep_their_own_state(fake):
+    """Batches of many signatures at once, sound and refused ones: every thread reads its own error,
+    and the tile choices they store in common are complete."""
+    fake(r'''
+import threading
+lib.cudapcgB200BatchLastError.restype = ctypes.c_char_p
+wrong = []
+def batch(shape, nmat):
+    n = int(np.prod(shape))
+    keys, nmats, K, CB = np.zeros(n, np.uint16), np.array([nmat], np.uint32), np.ones(256), np.ones(96)
+    one = lambda v: (ctypes.c_void_p * 1)(v.ctypes.data)
+    m, its, res = np.zeros(9), np.zeros(3, np.uint32), np.zeros(3)
+    rc = lib.cudapcgB200SolveThermalBatch(ctypes.c_uint(1), P(np.array([shape], np.uint32)), one(keys), P(nmats), one(K), one(CB),
+                                          ctypes.c_double(1e-6), ctypes.c_uint(10), 0, 1, P(m), P(its), P(res), None)
+    return rc, lib.cudapcgB200BatchLastError()
+def work(t):
+    for i in range(40):
+        rc, err = batch((2 + t, 3 + i, 4), 1)
+        if not rc or err: wrong.append((rc, err))
+        rc, err = batch((2 + t, 3 + i, 4), 9)
+        if rc or b"materials" not in err: wrong.append((rc, err))
+threads = [threading.Thread(target=work, args=(t,)) for t in range(8)]
+[t.start() for t in threads]; [t.join() for t in threads]
+assert not wrong, wrong[:3]
+''')
