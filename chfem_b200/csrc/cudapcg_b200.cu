@@ -496,7 +496,7 @@ static int pw_grid(long n) {
 // Largest grid any pass of the current model launches (reduction partials are sized once,
 // before graph capture, which must not allocate).
 static int needed_blocks() {
-  long nb = pw_grid(S->fluid ? S->nV + S->nB : S->N);
+  long nb = pw_grid(S->fluid ? S->nvars : S->N);  // Stokes: the pointwise passes run over unknowns
   // stencil passes: at most 8 resident CTAs of TE_NT = 256 threads per SM
   if (!S->fluid) nb = std::max<long>(nb, 8L * num_sms());
   return (int)nb;

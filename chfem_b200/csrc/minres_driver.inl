@@ -20,7 +20,8 @@ static MrCfg mrcfg() {
 static bool fl_by_node(int nr) { return S->N <= 4l * (S->nV + S->nB) && 32l * S->N * nr <= 16l << 30; }
 static size_t fl_record_bytes(int nr) { return 32ul * nr * std::max(fl_by_node(nr) ? S->N : S->nV + S->nB, 1l); }
 
-// The Stokes passes (stencil_fluid_mr.cuh) on explicit buffers, nr directions n unknowns apart.
+// The Stokes passes (stencil_fluid_mr.cuh) on explicit buffers, nr directions n unknowns apart.  A
+// pixel model solves one direction at a time: its blocks do not exist.
 static FlMrArgs fl_mr_args(int nr, double* r, double* q, double* s, double* d, double* x, double* z, int fin, bool skip_if_done) {
   return FlMrArgs{r, q, s, d, x, z, S->d_node_of_dof, S->d_bkeys, fl_by_node(nr) ? nullptr : S->d_dof_of_node, S->R, S->C, S->L, S->nV, S->nB, S->nvars,
                   S->cur_sc, RedCtl{}, mrcfg(), fin, skip_if_done};
@@ -30,16 +31,18 @@ static bool launch_fl_mr_dir(FlMrArgs a) {
   const int g = pw_grid(S->nvars);
   if (!ensure_reduction(g)) return false;
   a.rc = redctl(g);
-  if (S->fdim == 2) k_fl_mr_dir<NR, 2><<<g, PW_NT, 0, S->stream>>>(a);
-  else k_fl_mr_dir<NR, 3><<<g, PW_NT, 0, S->stream>>>(a);
+  if constexpr (NR == 1)
+    if (S->fdim == 2) k_fl_mr_dir<1, 2><<<g, PW_NT, 0, S->stream>>>(a);
+  if (S->fdim == 3) k_fl_mr_dir<NR, 3><<<g, PW_NT, 0, S->stream>>>(a);
   S->launches++;
   return cudaPeekAtLastError() == cudaSuccess;
 }
 template <int NR>
 static bool launch_fl_mr_upd(const FlMrArgs& a) {
   const int g = pw_grid(S->nvars);
-  if (S->fdim == 2) k_fl_mr_upd<NR, 2><<<g, PW_NT, 0, S->stream>>>(a);
-  else k_fl_mr_upd<NR, 3><<<g, PW_NT, 0, S->stream>>>(a);
+  if constexpr (NR == 1)
+    if (S->fdim == 2) k_fl_mr_upd<1, 2><<<g, PW_NT, 0, S->stream>>>(a);
+  if (S->fdim == 3) k_fl_mr_upd<NR, 3><<<g, PW_NT, 0, S->stream>>>(a);
   S->launches++;
   return cudaPeekAtLastError() == cudaSuccess;
 }
@@ -54,8 +57,9 @@ static bool launch_fl_mr_apply(FlMrArgs a) {
   if (!ensure_reduction(g)) return false;
   a.rc = redctl(g);
   const bool grid = !a.dof_of_node;
-  if (S->fdim == 2) grid ? launch_fl_mr_apply_dim<NR, 2, true>(a, g) : launch_fl_mr_apply_dim<NR, 2, false>(a, g);
-  else grid ? launch_fl_mr_apply_dim<NR, 3, true>(a, g) : launch_fl_mr_apply_dim<NR, 3, false>(a, g);
+  if constexpr (NR == 1)
+    if (S->fdim == 2) grid ? launch_fl_mr_apply_dim<1, 2, true>(a, g) : launch_fl_mr_apply_dim<1, 2, false>(a, g);
+  if (S->fdim == 3) grid ? launch_fl_mr_apply_dim<NR, 3, true>(a, g) : launch_fl_mr_apply_dim<NR, 3, false>(a, g);
   S->launches++;
   return cudaPeekAtLastError() == cudaSuccess;
 }
