@@ -1,11 +1,9 @@
-// modal_apply.cu -- launches of the operator passes in voxel modes (stencil_modal.cuh), and their
-// table.
+// modal_apply.cu -- the table of the passes in voxel modes (stencil_modal.cuh); their launches are in
+// modal_unit.cu.
 #include <algorithm>
 #include <cmath>
 #include <vector>
 #include "modal_apply.h"
-#include "device_cfg.h"
-#include "stencil_modal.cuh"
 #include "modal_point.cuh"
 
 namespace chfem {
@@ -93,111 +91,8 @@ bool md_build_table(int nd, int nmat, const double* Kd, double* tab) {
   return true;
 }
 
-namespace {
-// CTAs per SM the registers are capped for: as many as fit without spills (stencil_modal.cuh).
-template <int ND, typename V>
-constexpr int md_minb = ND == 1 ? (sizeof(V) == 8 ? 3 : 4) : (sizeof(V) == 8 ? 1 : 2);
-template <int ND, typename V, int MODE, bool BLK, bool DENS>
-constexpr auto md_kernel = k_modal_apply<ND, V, MODE, md_minb<ND, V>, BLK, DENS>;
-
-// CTAs of one pass: as many as fit on the GPU at once, but 8 layers of a tile each at least while
-// that leaves one per SM -- a CTA's fixed cost (table, first planes, its share of the reduction)
-// outweighs fewer layers: thermal 64^3 FP64 14.8 us at 148 CTAs, 18.0 at 444.
-template <int ND, typename V, int MODE, bool BLK, bool DENS>
-int ctas_of(int groups, int R, int C, int L, int num_sms) {
-  const size_t smem = md_smem_bytes<ND, V>();
-  static PerDevice kept;
-  const int per_sm = ctas_per_sm(kept, md_kernel<ND, V, MODE, BLK, DENS>, MD_NT, smem);
-  if (!per_sm) return 0;
-  const long work = (long)groups * ((R + TE_TR - 1) / TE_TR) * ((C + MD_TC - 1) / MD_TC) * L;
-  const long want = std::min(work, std::max((long)num_sms, work / 8));
-  return (int)std::max((long)groups, std::min((long)per_sm * num_sms, want));
-}
-template <int ND, typename V, int MODE, bool BLK, bool DENS>
-cudaError_t launch(const MdArgs<ND, typename MdV<V>::T>& a, int nb, cudaStream_t st) {
-  md_kernel<ND, V, MODE, BLK, DENS><<<nb, MD_NT, md_smem_bytes<ND, V>(), st>>>(a);
-  return cudaGetLastError();
-}
-}  // namespace
-
-template <int ND, typename T, int MODE>
-int md_ctas(bool density, int R, int C, int L, int num_sms) {
-  return density ? ctas_of<ND, T, MODE, false, true>(1, R, C, L, num_sms) : ctas_of<ND, T, MODE, false, false>(1, R, C, L, num_sms);
-}
-template <int ND, typename T, int MODE>
-cudaError_t md_launch(const TeArgs<ND, T>& a, const T* tab, int nb, cudaStream_t st) {
-  const MdArgs<ND, T> ma{a, tab, 0, 1};
-  return a.sdf ? launch<ND, T, MODE, false, true>(ma, nb, st) : launch<ND, T, MODE, false, false>(ma, nb, st);
-}
-
-// A pair of right-hand sides per CTA where their number is even and the fields are FP32 (packed
-// FP32 arithmetic), else one.
-template <int ND, typename T>
-int md_block_ctas(int nr, int R, int C, int L, int num_sms) {
-  if constexpr (sizeof(T) == 4) {
-    if (nr % 2 == 0) return ctas_of<ND, float2, TE_PCG, true, false>(nr / 2, R, C, L, num_sms);
-  }
-  return ctas_of<ND, T, TE_PCG, true, false>(nr, R, C, L, num_sms);
-}
-template <int ND, typename T>
-cudaError_t md_block_launch(int nr, long n, const TeArgs<ND, T>& a, const T* tab, int nb, cudaStream_t st) {
-  const MdArgs<ND, T> ma{a, tab, n, nr};
-  if constexpr (sizeof(T) == 4) {
-    if (nr % 2 == 0) return launch<ND, float2, TE_PCG, true, false>(ma, nb, st);
-  }
-  return launch<ND, T, TE_PCG, true, false>(ma, nb, st);
-}
-
-#define CHFEM_MD_INSTANTIATE(ND, T, MODE)                 \
-  template int md_ctas<ND, T, MODE>(bool, int, int, int, int); \
-  template cudaError_t md_launch<ND, T, MODE>(const TeArgs<ND, T>&, const T*, int, cudaStream_t);
-#define CHFEM_MD_MODES(ND, T)           \
-  CHFEM_MD_INSTANTIATE(ND, T, TE_PLAIN) \
-  CHFEM_MD_INSTANTIATE(ND, T, TE_PCG)   \
-  CHFEM_MD_INSTANTIATE(ND, T, TE_MR)    \
-  CHFEM_MD_INSTANTIATE(ND, T, TE_DIRDOT) \
-  CHFEM_MD_INSTANTIATE(ND, T, TE_UPD)
-CHFEM_MD_MODES(1, float)
-CHFEM_MD_MODES(1, double)
-CHFEM_MD_MODES(3, float)
-CHFEM_MD_MODES(3, double)
-#define CHFEM_MD_BLOCK(ND, T)                            \
-  template int md_block_ctas<ND, T>(int, int, int, int, int); \
-  template cudaError_t md_block_launch<ND, T>(int, long, const TeArgs<ND, T>&, const T*, int, cudaStream_t);
-CHFEM_MD_BLOCK(1, float)
-CHFEM_MD_BLOCK(1, double)
-CHFEM_MD_BLOCK(3, float)
-CHFEM_MD_BLOCK(3, double)
-
 // CTAs of 256 threads: 4 per SM keep enough 16-byte loads in flight for the memory's latency and
 // the partials that the last CTA sums few.
 int md_point_ctas(long n, int num_sms) { return (int)std::max(1L, std::min(4L * num_sms, (n / 2 + MP_NT - 1) / MP_NT)); }
-
-namespace {
-template <int ND, typename T, int NR, int VW>
-void point(const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st) {
-  if (norms) k_md_point<ND, T, NR, 2, VW><<<nb, MP_NT, 0, st>>>(a);
-  else if (parity) k_md_point<ND, T, NR, 1, VW><<<nb, MP_NT, 0, st>>>(a);
-  else k_md_point<ND, T, NR, 0, VW><<<nb, MP_NT, 0, st>>>(a);
-}
-template <int ND, typename T, int NR>
-void point_width(const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st) {
-  constexpr int FULL = 16 / (int)sizeof(T);
-  if (NR == 1 || a.n % FULL == 0) point<ND, T, NR, FULL>(a, parity, norms, nb, st);
-  else if (FULL == 4 && a.n % 2 == 0) point<ND, T, NR, 2>(a, parity, norms, nb, st);
-  else point<ND, T, NR, 1>(a, parity, norms, nb, st);
-}
-}  // namespace
-template <int ND, typename T>
-cudaError_t md_point_launch(int nr, const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st) {
-  if (nr == 1) point_width<ND, T, 1>(a, parity, norms, nb, st);
-  else if (nr == 3) point_width<ND, T, 3>(a, parity, norms, nb, st);
-  else if constexpr (ND == 3) point_width<ND, T, 6>(a, parity, norms, nb, st);
-  return cudaGetLastError();
-}
-template cudaError_t md_point_launch<1, float>(int, const MdPw<float>&, int, bool, int, cudaStream_t);
-template cudaError_t md_point_launch<1, double>(int, const MdPw<double>&, int, bool, int, cudaStream_t);
-template cudaError_t md_point_launch<3, float>(int, const MdPw<float>&, int, bool, int, cudaStream_t);
-template cudaError_t md_point_launch<3, double>(int, const MdPw<double>&, int, bool, int, cudaStream_t);
 
 }  // namespace chfem

@@ -1,5 +1,5 @@
-// modal_apply.h -- host entry of the operator passes in voxel modes (stencil_modal.cuh), compiled
-// in their own translation unit (modal_apply.cu).
+// modal_apply.h -- host entry of the passes in voxel modes (stencil_modal.cuh), compiled in their own
+// translation units (modal_unit.cu, modal_apply.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include "stencil_te.cuh"
@@ -16,10 +16,18 @@ inline bool md_layer_fits(int nd, long R, long C) { return R * C * nd * 8 < 0xff
 
 // CTAs of one pass (density: under a scalar density field, a.sdf) and one launch, with the
 // contract of k_te_apply<ND, T, MODE>.
+template <int ND, typename T, int MODE, bool DENS>
+int md_pass_ctas(int R, int C, int L, int num_sms);
+template <int ND, typename T, int MODE, bool DENS>
+cudaError_t md_pass_launch(const TeArgs<ND, T>& a, const T* tab, int nb, cudaStream_t st);
 template <int ND, typename T, int MODE>
-int md_ctas(bool density, int R, int C, int L, int num_sms);
+int md_ctas(bool density, int R, int C, int L, int num_sms) {
+  return density ? md_pass_ctas<ND, T, MODE, true>(R, C, L, num_sms) : md_pass_ctas<ND, T, MODE, false>(R, C, L, num_sms);
+}
 template <int ND, typename T, int MODE>
-cudaError_t md_launch(const TeArgs<ND, T>& a, const T* tab, int nb, cudaStream_t st);
+cudaError_t md_launch(const TeArgs<ND, T>& a, const T* tab, int nb, cudaStream_t st) {
+  return a.sdf ? md_pass_launch<ND, T, MODE, true>(a, tab, nb, st) : md_pass_launch<ND, T, MODE, false>(a, tab, nb, st);
+}
 
 // The block PCG operator pass on nr right-hand sides (contract of k_blk_apply); a: the fields of
 // the first of them (in0 = r, in1 = d_old, vout = d_new, y = q), n unknowns apart.
@@ -35,6 +43,12 @@ template <typename T>
 struct MdPw;
 int md_point_ctas(long n, int num_sms);
 template <int ND, typename T>
-cudaError_t md_point_launch(int nr, const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st);
+cudaError_t md_point_single(const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st);
+template <int ND, typename T>
+cudaError_t md_point_block(int nr, const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st);
+template <int ND, typename T>
+cudaError_t md_point_launch(int nr, const MdPw<T>& a, int parity, bool norms, int nb, cudaStream_t st) {
+  return nr == 1 ? md_point_single<ND, T>(a, parity, norms, nb, st) : md_point_block<ND, T>(nr, a, parity, norms, nb, st);
+}
 
 }  // namespace chfem

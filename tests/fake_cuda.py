@@ -15,7 +15,8 @@ import subprocess
 from tests import helpers as H
 
 OBJ = os.path.join(H.ROOT, "chfem_b200", "lib", "obj")
-OBJECTS = [os.path.join(OBJ, o + ".o") for o in ("cudapcg_b200", "modal_apply", "asm_apply", "pore_maps", "batch_thermal", "learned")]
+OBJECTS = [os.path.join(OBJ, o + ".o") for o in ("cudapcg_b200", "modal_apply", "asm_apply", "pore_maps", "batch_thermal", "learned")] + [
+    os.path.join(OBJ, f"modal_{n}_{t}_{p}.o") for n in (1, 3) for t in ("float", "double") for p in ("PASS", "DENSITY", "BLOCK", "POINT")]
 
 SOURCE = r'''
 #include <cstddef>

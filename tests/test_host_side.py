@@ -282,3 +282,10 @@ threads = [threading.Thread(target=work, args=(t,)) for t in range(8)]
 [t.start() for t in threads]; [t.join() for t in threads]
 assert not wrong, wrong[:3]
 ''')
+
+
+def test_single_passes_are_small_modules():
+    """The first launch of a kernel loads its whole module: the passes of one right-hand side are kept
+    apart from each other's field types and from the blocks', a megabyte or less each."""
+    sizes = {o: os.path.getsize(o) for o in fake_cuda.OBJECTS if o.endswith(("_PASS.o", "_DENSITY.o", "_POINT.o"))}
+    assert len(sizes) == 12 and max(sizes.values()) < 1.2e6, sizes
