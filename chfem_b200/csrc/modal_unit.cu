@@ -20,17 +20,22 @@ constexpr int md_minb = ND == 1 ? (sizeof(V) == 8 ? 3 : 4) : (sizeof(V) == 8 ? 1
 template <int ND, typename V, int MODE, bool BLK, bool DENS>
 constexpr auto md_kernel = k_modal_apply<ND, V, MODE, md_minb<ND, V>, BLK, DENS>;
 
-// CTAs of one pass: as many as fit on the GPU at once, but 8 layers of a tile each at least while
-// that leaves one per SM -- a CTA's fixed cost (table, first planes, its share of the reduction)
-// outweighs fewer layers: thermal 64^3 FP64 14.8 us at 148 CTAs, 18.0 at 444.
+// CTAs of one pass: as many as fit on the GPU at once, but 8 layers of a tile each at least -- a CTA's
+// fixed cost (table, first planes, its share of the reduction) outweighs fewer -- while that leaves
+// the SMs a CTA each, or two in the passes of (P)MINRES and the 3-vector PCG (whose layers wait on
+// more loads) and in models of more tiles than SMs (whose runs would cross tiles and restage planes).
+// Thermal FP64, us between events around a launch, one per SM against two: PCG pass 64^3 14.6 and
+// 14.7 (three: 15.3), 4 x 256 x 256 18.8 and 14.7; (P)MINRES pass 64^3 22.8 and 21.4, 4 x 256 x 256
+// 28.3 and 22.0.  The 3-vector PCG, both passes: 64^3 29.2 and 27.0 us an iteration.
 template <int ND, typename V, int MODE, bool BLK, bool DENS>
 int ctas_of(int groups, int R, int C, int L, int num_sms) {
   const size_t smem = md_smem_bytes<ND, V>();
   static PerDevice kept;
   const int per_sm = ctas_per_sm(kept, md_kernel<ND, V, MODE, BLK, DENS>, MD_NT, smem);
   if (!per_sm) return 0;
-  const long work = (long)groups * ((R + TE_TR - 1) / TE_TR) * ((C + MD_TC - 1) / MD_TC) * L;
-  const long want = std::min(work, std::max((long)num_sms, work / 8));
+  const long tiles = (long)groups * ((R + TE_TR - 1) / TE_TR) * ((C + MD_TC - 1) / MD_TC), work = tiles * L;
+  constexpr long least = MODE == TE_MR || MODE == TE_DIRDOT || MODE == TE_UPD ? 2 : 1;
+  const long want = std::min(work, std::max({least * num_sms, std::min(tiles, 2L * num_sms), work / 8}));
   return (int)std::max((long)groups, std::min((long)per_sm * num_sms, want));
 }
 template <int ND, typename V, int MODE, bool BLK, bool DENS>

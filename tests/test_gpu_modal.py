@@ -30,7 +30,7 @@ def both(monkeypatch, analysis, fn):
     return out
 
 
-SPECS = [((1, 1, 1), 1), ((1, 2, 3), 2), ((9, 33, 31), 2), ((3, 32, 8), 3), ((33, 7, 65), 2), ((4, 64, 10), 4)]
+SPECS = [((1, 1, 1), 1), ((1, 2, 3), 2), ((9, 33, 31), 2), ((3, 32, 8), 3), ((33, 7, 65), 2), ((4, 64, 10), 4), ((3, 70, 700), 2)]  # the last: more tiles than SMs
 
 
 @pytest.mark.parametrize("shape,nmat", SPECS)
@@ -58,7 +58,8 @@ def test_apply_equals_general_pass(tmp_path, monkeypatch, analysis, shape, nmat,
 
 @pytest.mark.parametrize("density", [False, True])
 @pytest.mark.parametrize("solver,norm", [(0, 0), (0, 1), (0, 2), (1, 0), (1, 2), (2, 0), (2, 2)])
-@pytest.mark.parametrize("analysis,shape,nmat", [(0, (9, 33, 12), 2), (0, (4, 10, 35), 4), (1, (5, 33, 9), 2), (1, (7, 8, 34), 3)])
+@pytest.mark.parametrize("analysis,shape,nmat", [(0, (9, 33, 12), 2), (0, (4, 10, 35), 4), (1, (5, 33, 9), 2), (1, (7, 8, 34), 3),
+                                                 (0, (2, 40, 650), 2)])
 def test_solve_equals_general_pass(tmp_path, monkeypatch, analysis, shape, nmat, solver, norm, density):
     """Every operator mode and both pointwise forms (x in every pass or in every second one), with
     iteration counts of either parity."""
