@@ -146,20 +146,21 @@ def setup_cudapcg_model(lib, arrays):
     """Drive the cudapcg C ABI of `lib` with host-layer arrays: init, model, maps, local matrices.
 
     arrays: dict with nx, ny, nz, N, ndof, nV, nB, nkeys, analysis (0/1/2), keys, dof_of_node,
-    node_of_dof, border, lcl (the formats of the cudapcg ABI)."""
+    node_of_dof, border, lcl (the formats of the cudapcg ABI), and dim2 for a pixel image."""
     a = arrays
-    an = {0: 1, 1: 3, 2: 5}[a["analysis"]]
+    dim2 = a.get("dim2", False)
+    an = {0: 1, 1: 3, 2: 5}[a["analysis"]] - dim2
     assert lib.cudapcgInit(an, 0)
     lib.cudapcgNewModel.restype = ctypes.POINTER(CudapcgModel)
     m = lib.cudapcgNewModel()
     mm = m.contents
-    mm.nrows, mm.ncols, mm.nlayers = a["ny"], a["nx"], a["nz"]
+    mm.nrows, mm.ncols, mm.nlayers = a["ny"], a["nx"], 0 if dim2 else a["nz"]
     mm.nelem = a["N"]
     mm.nvars = a["ndof"]
     mm.nkeys = a["nkeys"]
     mm.localmtxdim = a["lcl"].size // a["nkeys"]
     mm.nporenodes, mm.nbordernodes = a["nV"], a["nB"]
-    mm.nhmgvars = 3 * a["nV"] if a["analysis"] == 2 else a["ndof"]
+    mm.nhmgvars = (3 - dim2) * a["nV"] if a["analysis"] == 2 else a["ndof"]
     mm.poremap_flag = 1
     assert lib.cudapcgSetModel(m)
     import numpy as np

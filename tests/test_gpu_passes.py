@@ -2,7 +2,8 @@
 
 Oracles: an extruded image of one layer solved by the 3D passes for any matrix has the tensor of its
 2D image (the solution does not depend on z); a Stokes solution's residual through the operator
-gathered by DOF number (cudapcgB200ApplyOperator), which the (P)MINRES passes do not use.
+gathered by DOF number (cudapcgB200ApplyOperator), which the (P)MINRES passes do not use, for voxels
+and pixels; a Stokes block (voxels only) against its directions one by one.
 """
 import ctypes
 import zlib
@@ -40,7 +41,7 @@ def stokes_case(tmp_path, shape, porosity):
     img = np.where(rng.random(shape) < porosity, 0, 255).astype(np.uint8)
     if porosity < 0:  # a duct: more than four nodes per fluid node, the records by DOF number
         img[:] = 255
-        img[:, 4:10, 5:11] = 0
+        img[..., 4:10, 5:11] = 0
     elif len(shape) == 3 and min(shape) > 8:  # connected pores: a smooth field
         from chfem_b200.synthetic import pore_grf
         img = pore_grf(shape, corr=2.0, porosity=porosity, seed=5)
@@ -49,11 +50,11 @@ def stokes_case(tmp_path, shape, porosity):
 
 @pytest.mark.parametrize("precondition", [0, 1])
 @pytest.mark.parametrize("shape,porosity", [((3, 3, 3), 1.0), ((5, 6, 7), 0.9), ((9, 33, 10), 0.6), ((17, 12, 35), 0.45),
-                                            ((24, 20, 28), -1)])
+                                            ((24, 20, 28), -1), ((3, 4), 1.0), ((25, 21), 0.75), ((40, 33), 0.7), ((31, 28), -1)])
 def test_stokes_solution_meets_its_tolerance(tmp_path, shape, porosity, precondition):
     from chfem_b200 import _native
     img, (nf, raw) = stokes_case(tmp_path, shape, porosity)
-    a = host_arrays(nf, raw)
+    a = dict(host_arrays(nf, raw), dim2=len(shape) == 2)
     lib = _native.cudapcg()
     p = lambda v: v.ctypes.data_as(ctypes.c_void_p)
     lib.cudapcgGetResidual.restype = ctypes.c_double
@@ -78,12 +79,12 @@ def test_stokes_solution_meets_its_tolerance(tmp_path, shape, porosity, precondi
     else:
         rel = np.linalg.norm(r) / np.linalg.norm(b)
     lib.cudapcgEnd()
-    # the recurrence's residual norm stops the solve; the true one drifts from it by round-off
-    assert rel < 20 * tol, rel
+    # the recurrence's residual stops the solve at tol; the true one drifts from it by FP64 round-off,
+    # far below tol (at most 0.998 tol over these cases with three right-hand sides each)
+    assert rel < 1.01 * tol, rel
 
 
-@pytest.mark.parametrize("shape,porosity", [((6, 7, 9), 0.9), ((12, 33, 10), 0.6), ((25, 21), 0.75), ((40, 33), 0.7),
-                                            ((24, 20, 28), -1)])
+@pytest.mark.parametrize("shape,porosity", [((6, 7, 9), 0.9), ((12, 33, 10), 0.6), ((24, 20, 28), -1)])
 def test_stokes_block_equals_single_cases(tmp_path, shape, porosity):
     from chfem_b200 import compute_property
     img, _ = stokes_case(tmp_path, shape, porosity)
