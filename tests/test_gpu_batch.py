@@ -124,12 +124,12 @@ def test_batch_of_isotropic_materials_equals_any_matrices(tmp_path, sizes, preci
             ctypes.c_double(1e-10 if precision == 0 else 1e-7), ctypes.c_uint(5000), precision, precondition,
             moments.ctypes.data_as(ctypes.c_void_p), its.ctypes.data_as(ctypes.c_void_p), res.ctypes.data_as(ctypes.c_void_p), None)
         assert rc == 1, lib.cudapcgB200BatchLastError()
+        # the residual that ended each case: in mixed precision the true one of the FP64 solution
+        assert (res <= 1.000001 * (1e-10 if precision == 0 else 1e-7)).all() and (its < 5000).all(), (res, its)
         out.append((moments, its.astype(int)))
     (m0, i0), (m1, i1) = out
     assert H.rel_to_max(m0, m1) < (1e-8 if precision == 0 else 1e-4)
+    # mixed: 1e-7 is at the rounding of FP32 (6e-8), where a case goes on after its check or not, so
+    # that counts differ by whole restart cycles; what binds them is the residual above
     if precision == 0:
         assert np.abs(i0 - i1).max() <= 1, (i0, i1)
-    else:
-        # 1e-7 is at the rounding of FP32 (6e-8): a case passes its test on the recursive residual,
-        # fails the check on the true one and goes on, whole restart cycles later or not
-        assert all(a <= 2 * b + 50 and b <= 2 * a + 50 for a, b in zip(i0, i1)), (i0, i1)

@@ -241,9 +241,8 @@ def test_operator_and_jacobi(tmp_path, name, analysis, spec, precision):
 @pytest.mark.parametrize("spec", [("img", (13, 35, 17), 4), ("img", (40, 9, 66), 2), ("img", (1, 2, 3), 3)])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_thermal_pass_equals_generic(tmp_path, spec, precision, monkeypatch):
-    """The thermal pass written for cubic-symmetric conduction matrices (stencil_th.cuh) against
-    the oracle and against the generic thermal pass (CHFEM_B200_THERMAL_OP=generic), 2 to 4
-    materials, thin and ragged shapes."""
+    """The thermal pass in voxel modes (stencil_modal.cuh) against the oracle and against the generic
+    thermal pass (CHFEM_B200_THERMAL_OP=generic), 2 to 4 materials, thin and ragged shapes."""
     import pickle
     from chfem_b200 import _native
     nf, raw = build_small(tmp_path, "thp", 0, spec)
@@ -287,9 +286,9 @@ np.save(sys.argv[1] + ".ys.npy", np.array(ys))
 '''
 
 
-# The block operator pass of the block solver (for one- and two-material models the stencil
-# assembled per material configuration, otherwise element by element), applied to 3 or 6
-# random fields at once; each output against the oracle's single apply.  Bars as above.
+# The block operator pass of the block solver (in voxel modes: these materials are isotropic; the
+# passes for any matrices are in test_gpu_assembled.py), applied to 3 or 6 random fields at once;
+# each output against the oracle's single apply.  Bars as above.
 @pytest.mark.parametrize("name,analysis,spec,nr", [
     ("th2", 0, ("img", (13, 35, 17), 2), 3), ("th1", 0, ("img", (9, 8, 11), 1), 3), ("th3", 0, ("img", (10, 33, 9), 3), 3),
     ("el2", 1, ("img", (9, 33, 10), 2), 6), ("el2_3", 1, ("img", (11, 7, 13), 2), 3), ("el4", 1, ("img", (7, 9, 8), 4), 6),
