@@ -65,6 +65,46 @@ def oracle_available():
     return os.path.exists(ORACLE_EXEC) and os.path.exists(ORACLE_REF_LIB)
 
 
+def conductivity_tensor(img, props, tol=1e-10):
+    """Effective conductivity of a periodic (z, y, x) image on trilinear voxels, in NumPy: the oracle
+    where the other is not built.  A corrector per unit gradient by conjugate gradients;
+    C_ij = mean of k (X_i + chi_i)^T K (X_j + chi_j) over the voxels; y and z run against the
+    image's axes."""
+    img = np.asarray(img)[::-1, ::-1]
+    k = np.zeros(img.shape)
+    for c, v in props.items():
+        k[img == c] = v
+    corners = [(z, y, x) for z in (0, 1) for y in (0, 1) for x in (0, 1)]
+    at = np.array(corners)
+    same = at[:, None, :] == at[None, :, :]
+    S, M = np.where(same, 1.0, -1.0), np.where(same, 1 / 3, 1 / 6)  # 1D stiffness and mass
+    K = sum(S[..., i] * M[..., (i + 1) % 3] * M[..., (i + 2) % 3] for i in range(3))
+
+    def gather(u):
+        return np.stack([np.roll(u, [-a for a in c], (0, 1, 2)) for c in corners])
+
+    def scatter(f):
+        return sum(np.roll(f[n], c, (0, 1, 2)) for n, c in enumerate(corners))
+    apply = lambda u: scatter(k * np.einsum("ab,b...->a...", K, gather(u)))
+    us = []
+    for axis in (2, 1, 0):  # x, y, z
+        X = at[:, axis].astype(float)
+        r = -scatter(k * (K @ X)[:, None, None, None])
+        chi, d, rr = np.zeros(img.shape), r.copy(), (r * r).sum()
+        stop = tol * tol * rr
+        for _ in range(20 * img.size):
+            if rr <= stop:
+                break
+            q = apply(d)
+            alpha = rr / (d * q).sum()
+            chi += alpha * d
+            r -= alpha * q
+            rr, old = (r * r).sum(), rr
+            d = r + rr / old * d
+        us.append(gather(chi) + X[:, None, None, None])
+    return np.array([[(k * (u * np.einsum("ab,b...->a...", K, v)).sum(axis=0)).mean() for v in us] for u in us])
+
+
 # ---- oracle captures, computed in a child process -------------------------------------
 _CAPTURE_SCRIPT = r'''
 import ctypes, sys, json, numpy as np
@@ -102,6 +142,9 @@ np.savez(out, **arrs)
 def oracle_capture(nf, raw, direction):
     """Run the reference host code + CPU oracle solver on one load case; returns the arrays the
     host code handed over the cudapcg ABI (keys, maps, local matrices, RHS, solution) and C."""
+    if not os.path.exists(ORACLE_REF_LIB):
+        import pytest
+        pytest.skip("oracle/_ref not built (needs the reference tree)")
     out = tempfile.mktemp(suffix=".npz")
     p = subprocess.run([sys.executable, "-c", _CAPTURE_SCRIPT, ORACLE_REF_LIB, nf, raw, str(direction), out],
                        capture_output=True, text=True, timeout=1800, env=dict(os.environ, OMP_NUM_THREADS=str(os.cpu_count() or 4)))
