@@ -748,6 +748,18 @@ def rel_to_max(a, b):
     return float(np.abs(a - b).max() / max(np.abs(b).max(), 1e-300))
 
 
+def operator_passes(model, w, nd):
+    """Which operator passes a thermal or elastic model of isotropic phases runs on, by the library's
+    own rule: in voxel modes for up to four phases of positive conductivity or stiffness; else, or
+    where a variable deselects them, assembled by neighbour for two, element by element for more."""
+    values = [v if nd == 1 else v[0] for v in w["props"].values()]
+    element = os.environ.get("CHFEM_B200_BLOCK_OP") == "element"
+    deselected = os.environ.get("CHFEM_B200_THERMAL_OP") == "generic" if nd == 1 else element
+    if model.nmat <= 4 and min(values) > 0 and not deselected:
+        return "modal"
+    return "assembled" if model.nmat <= 2 and not element else "element"
+
+
 def dominant_kernel_roofline(model, w, block, workload):
     """The dominant kernel timed live on the library's stream (CUDA events around each launch),
     its algorithmic bytes per node against the measured HBM peak."""
@@ -764,21 +776,21 @@ def dominant_kernel_roofline(model, w, block, workload):
     else:
         nd = 3 if w["analysis"] == 1 else 1
         tn = 'float' if es == 4 else 'double'
+        passes = operator_passes(model, w, nd)
         if block:
             nr = 6 if nd == 3 else 3
-            modal = os.environ.get("CHFEM_B200_BLOCK_OP") != "element"
             kern_which = 5
             vt = "float2" if es == 4 and nr % 2 == 0 else tn
-            kname = (f"k_modal_apply<{nd},{vt},TE_PCG> block (operator in voxel modes + directions + dots, {nr} load cases)" if modal else
-                     f"k_blk_apply<{nd},{tn},{nr}> (block operator + directions + dots, {nr} load cases)")
-            per_unit = nr * 4 * nd * es + 2  # per load case s, d_old in; d_new, q out; one 16-bit key
-        elif os.environ.get("CHFEM_B200_THERMAL_OP" if nd == 1 else "CHFEM_B200_BLOCK_OP") not in ("generic", "element"):
-            kern_which = 1
-            kname = f"k_modal_apply<{nd},{tn},TE_PCG> (operator in voxel modes + direction + dot)"
-            per_unit = 4 * nd * es + 2
+            kname = {"modal": f"k_modal_apply<{nd},{vt},TE_PCG> block (operator in voxel modes + directions + dots, {nr} load cases)",
+                     "assembled": f"k_asm_apply<{nd},{tn},{nr}> (block operator assembled by neighbour + directions + dots, {nr} load cases)",
+                     "element": f"k_blk_apply<{nd},{tn},{nr}> (block operator + directions + dots, {nr} load cases)"}[passes]
+            per_unit = nr * 4 * nd * es + 2  # per load case r, d_old in; d_new, q out; one 16-bit key
         else:
-            kern_which, kname = 1, f"k_te_apply<{nd},{tn},TE_PCG> (operator + direction + dot)"
-            per_unit = 4 * nd * es + 2  # s, d_old in; d_new, q out (nd comps); 16-bit key
+            kern_which = 1
+            kname = {"modal": f"k_modal_apply<{nd},{tn},TE_PCG> (operator in voxel modes + direction + dot)",
+                     "assembled": f"k_te_apply<{nd},{tn},TE_PCG,true> (operator assembled by neighbour + direction + dot)",
+                     "element": f"k_te_apply<{nd},{tn},TE_PCG> (operator + direction + dot)"}[passes]
+            per_unit = 4 * nd * es + 2  # r, d_old in; d_new, q out (nd comps); 16-bit key
         units = model.N
     kt = model.kernel_time(kern_which, reps=30)
     achieved = per_unit * units / kt / 1e9 if kt > 0 else None
