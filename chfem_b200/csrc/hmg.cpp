@@ -944,7 +944,7 @@ int chfemB200ColorHistogram(const uint8_t* voxels, unsigned long long n, unsigne
 #pragma omp parallel if (n > (1u << 16))
   {
     // four tables taken in turn, so that a run of one colour does not wait on its own counter
-    std::vector<unsigned long long> h(4 * 256, 0);
+    unsigned long long h[4 * 256] = {0};  // on the stack: nothing here can throw
 #pragma omp for nowait
     for (long long i = 0; i < (long long)(n / 4); i++)
       for (int k = 0; k < 4; k++) h[256 * k + voxels[4 * i + k]]++;
