@@ -130,7 +130,7 @@ struct Batch {
   long* d_noff = nullptr;
   uint16_t* d_keys = nullptr;
   TV* d_K = nullptr;
-  bool iso = false;  // every conductivity matrix is isotropic
+  bool iso = false;  // every conductivity matrix is isotropic and positive
   double *d_K64 = nullptr, *d_CB = nullptr, *d_x = nullptr, *d_b = nullptr, *d_part = nullptr, *d_mom = nullptr;
   TV *d_r = nullptr, *d_s = nullptr, *d_d0 = nullptr, *d_d1 = nullptr, *d_q = nullptr;
   DevScalars* d_sc = nullptr;

@@ -63,7 +63,7 @@ struct BtData {
   const uint16_t* keys;      // [noff[n]]
   const TV* K;               // [n][4][64] dense conductivity matrices (slots past nmat zero)
   const double* K64;         // same in FP64 (replacement operator, right-hand sides)
-  int iso;                   // every conductivity matrix is isotropic (one diagonal value per material)
+  int iso;                   // every conductivity matrix is isotropic and positive (one diagonal value per material)
   DevScalars* sc;            // [n][3]
   BtCtl* ctl;                // [n][3]
   const BtSched* sch;

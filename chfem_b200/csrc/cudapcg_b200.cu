@@ -318,7 +318,7 @@ static bool ensure_vectors() {
 }
 
 // Assembled neighbour blocks (stencil_asm.cuh) of a thermal/elastic model of at most two
-// materials that are not isotropic; CHFEM_B200_BLOCK_OP=element keeps the element-by-element
+// materials that does not run in voxel modes; CHFEM_B200_BLOCK_OP=element keeps the element-by-element
 // operator.
 static bool md_applies();
 static bool asm_applies() {
@@ -345,8 +345,8 @@ static bool ensure_tab() {
 }
 
 // The passes in voxel modes (stencil_modal.cuh): 3D thermal and elastic models whose element
-// matrices are those of isotropic materials on cubes (checked once per model), the reference's
-// and this library's models.  CHFEM_B200_THERMAL_OP=generic (thermal) and
+// matrices are those of isotropic materials on cubes (checked once per model): the reference's and
+// this library's models whose phases all have a positive conductivity or stiffness.  CHFEM_B200_THERMAL_OP=generic (thermal) and
 // CHFEM_B200_BLOCK_OP=element (elastic) keep the passes that take any element matrix.
 static bool md_applies() {
   if (S->fluid || S->dim2 || S->nmat > 4 || !S->have_K || !md_layer_fits(S->nd, S->R, S->C)) return false;
@@ -520,7 +520,8 @@ static int d2_ctas() {
 template <int ND, typename T, int MODE>
 static bool launch_md(const T* in0, const T* in1, T* vout, T* y, double* x, const T* d, int finish, int skip_if_done, const MrCfg& cfg) {
   const int nb = md_ctas<ND, T, MODE>(S->d_sdf != nullptr, S->R, S->C, S->L, num_sms());
-  if (nb < 1 || !ensure_reduction(nb)) return false;
+  if (nb < 1) { set_err("operator pass", "launch configuration"); return false; }
+  if (!ensure_reduction(nb)) return false;
   TeArgs<ND, T> a{in0, in1, vout, y, x, d, S->d_keys, nullptr, S->nmat, S->R, S->C, S->L, S->cur_sc, redctl(nb), finish, skip_if_done, cfg};
   sdf_args(a);
   const cudaError_t e = md_launch<ND, T, MODE>(a, mddev<T>(), nb, S->stream);

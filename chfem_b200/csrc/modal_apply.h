@@ -8,7 +8,8 @@ namespace chfem {
 
 // The pass's table (md_table_words() values, FP64) from the dense element matrices of nmat <= 4
 // materials (Kd[m][8 nd][8 nd]); false when a matrix is not that of an isotropic material on a
-// cube (to 1e-12 of its largest entry), the structure the passes rely on.
+// cube (to 1e-12 of its largest entry), the structure the passes rely on, or its diagonal is not
+// positive (a node inside such a phase has no inverse diagonal).
 bool md_build_table(int nd, int nmat, const double* Kd, double* tab);
 int md_table_words();
 // whether the passes' 32-bit byte offsets in a layer hold a layer of R x C nodes
