@@ -1721,7 +1721,11 @@ extern "C" {
 template <typename T>
 static double time_kernel_T(int which, unsigned reps) {
   if (!ensure_vectors<T>() || !ensure_K<T>()) return -1.0;
-  if (!S->q || ((which == 1 || which == 2) && !S->d1) || ((which == 3 || which == 4) && !S->r2 && !S->fl_z)) { set_err("cudapcgB200TimeKernel", "kernel not used by the selected solver"); return -1.0; }
+  if (which == 1 || which == 2) {  // PCG's passes under another solver: its second direction buffer
+    if (!S->d1 && dev_malloc(&S->d1, (size_t)S->nvars * sizeof(T)) != cudaSuccess) { set_err("cudapcgB200TimeKernel", "device allocation failed"); return -1.0; }
+    if (cudaMemsetAsync(S->d1, 0, (size_t)S->nvars * sizeof(T), S->stream) != cudaSuccess) return -1.0;
+  }
+  if (!S->q || ((which == 3 || which == 4) && !S->r2 && !S->fl_z)) { set_err("cudapcgB200TimeKernel", "kernel not used by the selected solver"); return -1.0; }
   if (!ensure_reduction(needed_blocks())) return -1.0;
   // each repetition resets the scalars (so no pass exits early) and brackets only the launch
   float total = 0.f;
