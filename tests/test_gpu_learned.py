@@ -129,3 +129,20 @@ def test_network_at_tile_edges(shape):
     for name, (w0, b0, co, ci, k) in LO.offsets()[0].items():
         assert H.rel_to_max(g[w0:b0], gref[w0:b0]) < 1e-3, name
         assert H.rel_to_max(g[b0:b0 + co], gref[b0:b0 + co]) < 1e-3, name
+
+
+@pytest.mark.parametrize("multirhs", [True, False])
+def test_learned_guess_on_a_side_stream(multirhs):
+    """The guesses are made on the caller's current stream; the solve that reads them waits for it."""
+    import torch
+    from chfem_b200 import _native, compute_property, synthetic
+    img = synthetic.grf((16, 24, 32), corr=4.0, fraction=0.4, seed=7)
+    kw = dict(mat_props={0: (1.0, 0.30), 255: (20.0, 0.20)}, solver_tolerance=1e-6, multirhs=multirhs, initial_guess="learned")
+    runs = []
+    for stream in (torch.cuda.default_stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(40_000_000)  # some 20 ms of queued work before the guesses
+            C = np.array(compute_property("elasticity", img, **kw))
+        runs.append((C, list(_native.solve_stats().iterations)))
+    (C0, its0), (C1, its1) = runs
+    assert its0 == its1 and H.rel_to_max(C1, C0) < 1e-12
