@@ -96,9 +96,10 @@ def compute_property(property, array, mat_props=None, voxel_size=1e-6, solver=No
             raise ValueError("initial_guess='learned' needs refinement 1 and every axis divisible by 8")
         from . import learned
         guesses = learned.device_guesses(learned.default_net(), array, mat_props)
-        # the solver's uploads follow the legacy default stream, not the caller's current one
+        # the solver reads them after the legacy default stream's work: order that after the caller's
+        # current stream, without holding up the set-up on the host
         import torch
-        torch.cuda.current_stream().synchronize()
+        torch.cuda.default_stream().wait_stream(torch.cuda.current_stream())
     try:
         flat = np.ascontiguousarray(np.reshape(array, array.size), dtype=np.uint8)
         lib = _native.chfem()
